@@ -201,6 +201,11 @@ struct qagg_aggregator
     std::vector<QItem> iK1, iK2;
     long long k3Units = 0; // work units of the unquantize launch
     int k3SmemWords = 0;   // shared-memory words per warp the unquantize launch needs
+    // one rank: the unquantize table of the matrices that are quantized apart (hK1t), the only ones the quantize kernel
+    // does not expand itself
+    std::vector<QTensor> hK3t;
+    long long k3tUnits = 0;
+    QTensor* dK3t = nullptr;
     QTensor *dK1 = nullptr, *dK2 = nullptr, *dK3 = nullptr;
     QItem *dI1 = nullptr, *dI2 = nullptr;
     // consumer fusion: a copy of the unquantize table whose destinations are the caller's parameter and smoothed-gradient
@@ -216,7 +221,7 @@ struct qagg_aggregator
     struct Binding
     {
         std::vector<float*> grads;
-        QTensor *dK1 = nullptr, *dK2 = nullptr, *dK3 = nullptr, *dK1t = nullptr;
+        QTensor *dK1 = nullptr, *dK2 = nullptr, *dK3 = nullptr, *dK1t = nullptr, *dK3t = nullptr;
         QItem *dI1 = nullptr, *dI2 = nullptr, *dI1t = nullptr;
     };
     Binding bindings[2];
@@ -513,6 +518,15 @@ int build_tables(qagg_aggregator* a)
                 tallCols += n;
             }
         }
+        a->hK3t.clear();
+        a->k3tUnits = 0;
+        if (K == 1)
+            for (int i : a->k1tTensor)
+            {
+                a->hK3t.push_back(a->hK3[i]);
+                a->hK3t.back().unit0 = a->k3tUnits;
+                a->k3tUnits += unq_units(a->M[i], a->N[i], a->bits);
+            }
         if (!a->hK1t.empty())
         {
             int rc;
@@ -596,7 +610,7 @@ int build_tables(qagg_aggregator* a)
 
 size_t table_bytes(const qagg_aggregator* a)
 {
-    return (a->hK1.size() + a->hK2.size() + a->hK3.size() + a->hK1t.size()) * sizeof(QTensor) +
+    return (a->hK1.size() + a->hK2.size() + a->hK3.size() + a->hK1t.size() + a->hK3t.size()) * sizeof(QTensor) +
            (a->iK1.size() + a->iK2.size() + a->iK1t.size()) * sizeof(QItem) + 256;
 }
 
@@ -631,6 +645,8 @@ int upload_tables(qagg_aggregator* a, int slot)
         return rc;
     if ((rc = put(a->iK1t.data(), a->iK1t.size() * sizeof(QItem), (void**) &a->dI1t)))
         return rc;
+    if ((rc = put(a->hK3t.data(), a->hK3t.size() * sizeof(QTensor), (void**) &a->dK3t)))
+        return rc;
     return QAGG_OK;
 }
 
@@ -652,6 +668,7 @@ int bind_grads(qagg_aggregator* a, float* const* grads, cudaStream_t st)
             a->dI2 = b.dI2;
             a->dK1t = b.dK1t;
             a->dI1t = b.dI1t;
+            a->dK3t = b.dK3t;
             return QAGG_OK;
         }
     }
@@ -662,6 +679,7 @@ int bind_grads(qagg_aggregator* a, float* const* grads, cudaStream_t st)
         if (!grads[i] && a->M[i] * a->N[i] > 0)
             return fail(QAGG_EINVAL, "qagg_agg_step: null gradient pointer");
         a->hK1[i].grad = grads[i];
+        a->hK1[i].out = grads[i]; // one rank: the quantize kernel expands into the gradient (quantize_expands)
         a->hK3[i].out = grads[i];
     }
     const int r = a->comm->rank;
@@ -672,6 +690,8 @@ int bind_grads(qagg_aggregator* a, float* const* grads, cudaStream_t st)
     }
     for (size_t e = 0; e < a->hK1t.size(); ++e)
         a->hK1t[e].grad = grads[a->k1tTensor[e]] + a->k1tCol[e] * a->M[a->k1tTensor[e]];
+    for (size_t e = 0; e < a->hK3t.size(); ++e)
+        a->hK3t[e].out = grads[a->k1tTensor[e]];
     // an earlier step may still be reading the tables of that set -- on this stream or on the one it was enqueued on
     int rc = check_cuda(cudaStreamSynchronize(st), "cudaStreamSynchronize");
     if (rc)
@@ -700,6 +720,7 @@ int bind_grads(qagg_aggregator* a, float* const* grads, cudaStream_t st)
     b.dI2 = a->dI2;
     b.dK1t = a->dK1t;
     b.dI1t = a->dI1t;
+    b.dK3t = a->dK3t;
     a->curBinding = slot;
     return QAGG_OK;
 }
@@ -736,9 +757,17 @@ Signal make_signal(const qagg_aggregator* a, bool gatherPhase)
     }
     return sg;
 }
+// One rank: what it quantized is the aggregate, so the quantize kernel stores the unquantized values itself and the
+// unquantize launch, which would read every packed word back, is left out.  With the learner step bound the launch stays: it
+// is the kernel that applies the update.
+bool quantize_expands(const qagg_aggregator* a)
+{
+    return a->comm->K == 1 && !a->updating;
+}
 int launch_k1(qagg_aggregator* a, cudaStream_t st)
 {
     const Signal sg = make_signal(a, false);
+    const bool expand = quantize_expands(a);
     if (a->deferred && !a->hK1t.empty())
     {
         // Very tall matrices: formed first, then walked on this stream while the streaming kernel takes the other matrices on
@@ -754,8 +783,13 @@ int launch_k1(qagg_aggregator* a, cudaStream_t st)
         if ((rc = check_cuda(cudaStreamWaitEvent(a->k1Side, a->k1Fork, 0), "cudaStreamWaitEvent")))
             return rc;
         if (!a->iK1.empty() &&
-            (rc = check_cuda(launch_stream1(a->k1Side, a->dK1, a->dI1, (int) a->iK1.size(), a->cfg, static_cast<unsigned*>(a->queue.p), &quiet, a->status_word()),
+            (rc = check_cuda(launch_stream1(a->k1Side, a->dK1, a->dI1, (int) a->iK1.size(), a->cfg, static_cast<unsigned*>(a->queue.p), &quiet, a->status_word(),
+                                       expand),
                              "quantize launch")))
+            return rc;
+        // the tall matrices expand while the streaming kernel is still at the others
+        if (expand && (rc = check_cuda(launch_unquantize(st, UNQ_STORE, a->bits, nullptr, a->dK3t, (int) a->hK3t.size(), a->k3tUnits, a->k3SmemWords, a->cfg),
+                                       "unquantize launch (tall matrices)")))
             return rc;
         if ((rc = check_cuda(cudaEventRecord(a->k1Join, a->k1Side), "cudaEventRecord")) ||
             (rc = check_cuda(cudaStreamWaitEvent(st, a->k1Join, 0), "cudaStreamWaitEvent")))
@@ -763,10 +797,11 @@ int launch_k1(qagg_aggregator* a, cudaStream_t st)
         return sg.n > 0 ? check_cuda(launch_signal_only(st, sg), "flag release launch") : QAGG_OK;
     }
     if (a->deferred)
-        return check_cuda(launch_stream1(st, a->dK1, a->dI1, (int) a->iK1.size(), a->cfg, static_cast<unsigned*>(a->queue.p), &sg, a->status_word()),
+        return check_cuda(launch_stream1(st, a->dK1, a->dI1, (int) a->iK1.size(), a->cfg, static_cast<unsigned*>(a->queue.p), &sg, a->status_word(),
+                                         expand),
                           "quantize launch");
     return check_cuda(launch_colquant(st, false, a->mode, nullptr, a->dK1, a->dI1, (int) a->iK1.size(), 0, a->cfg,
-                                      static_cast<unsigned*>(a->queue.p), &sg), "quantize launch");
+                                      static_cast<unsigned*>(a->queue.p), &sg, expand), "quantize launch");
 }
 int launch_k2(qagg_aggregator* a, cudaStream_t st)
 {
@@ -807,6 +842,8 @@ int wait_peers(qagg_aggregator* a, bool gatherPhase, cudaStream_t st)
 }
 int launch_k3(qagg_aggregator* a, cudaStream_t st)
 {
+    if (quantize_expands(a))
+        return QAGG_OK;
     if (a->updating)
         return check_cuda(launch_unquantize(st, UNQ_UPDATE, a->bits, nullptr, static_cast<const QTensor*>(a->updTable.p), (int) a->hK3.size(), a->k3Units,
                                             a->k3SmemWords, a->cfg, &a->updRule), "unquantize-update launch");
@@ -2190,8 +2227,8 @@ int qagg_agg_launches_per_step(const qagg_aggregator* a)
         return fail(QAGG_EINVAL, "null aggregator");
     if (a->identity || a->totalValues == 0)
         return 0;
-    if (a->comm->K == 1)
-        return 2;
+    if (a->comm->K == 1) // quantize, or form + walk and the others' quantize; one more to unquantize what that did not expand
+        return (a->hK1t.empty() ? 1 : 2 + (a->iK1.empty() ? 0 : 1)) + ((quantize_expands(a) && a->hK1t.empty()) ? 0 : 1);
     // quantize, owner (one kernel, or form + walk, or both twice when the tall matrices go apart), unquantize; + two flag waits
     // (+ the gather push) (+ a header push when the last step carried a header that the quantize kernel did not take along)
     // in peer mode

@@ -6,18 +6,20 @@
 // Same arithmetic contract as the float kernels: every operation an explicit round-to-nearest double intrinsic, operand
 // types as the reference's (size_t -> double before divides, unsigned x double, truncating double -> int64), the float
 // literals 1e-36f / 0.5f / 2.0f / 4.0f promoted as the reference's template does, and every per-column sum accumulated in
-// ROW ORDER.  Layout: one CTA per column at a time; the column's values v = gradient + residual pass through shared
-// memory in chunks of 1024 rows, loaded by all threads; lane 0 of warp 0 walks the lower-level chain (or the single sum of
-// the other modes) and lane 0 of warp 1 the upper-level chain, both carrying their accumulators from chunk to chunk;
-// afterwards all threads quantize, one packed word each.  A plain kernel: the double path is a completeness row, not the
-// benchmarked one.
+// ROW ORDER.  A column's walk is a chain of M dependent double adds per level, so everything else is arranged around
+// having that chain run undisturbed: one CTA per column; all threads stage v = gradient + residual in shared memory and count
+// the rows below a threshold of 0; then lane 0 of warp 0 walks the lower level (or the single sum of the other modes) and
+// lane 0 of warp 1 the upper one, the next eight rows always loaded ahead of the adds; then all threads quantize.
 #include "../../include/qagg.h"
 #include "qagg_internal.h"
 
+#include <algorithm>
+
 namespace qagg {
 
-constexpr int DNT = 128;     // threads per CTA
-constexpr int DCHUNK = 1024; // rows per staged chunk
+constexpr int DRESIDENT = 24576; // most rows of a column that stays in shared memory (192 KB)
+constexpr int DCHUNK = 4096;     // rows per staged chunk of a taller one
+constexpr int DWORDS = 1024;     // packed words of a column that are assembled in shared memory
 
 struct ValQD
 {
@@ -69,85 +71,151 @@ __device__ __forceinline__ double unquantize_d(const ValQD& q, int bits, unsigne
     return __dadd_rn(__dmul_rn(__dadd_rn(__ull2double_rn(u), 0.5), q.ufactor), q.qmin);
 }
 
-// ComputeRangeStatColjSubset for one column (ColumnQuantizer.h:209-341) + Quantize (ColumnQuantizer.h:50-65, 90-147)
-__global__ void __launch_bounds__(DNT) k_quantize_f64(const double* __restrict__ grad, const double* __restrict__ resIn, double* __restrict__ resOut,
-                                                     unsigned char* __restrict__ packed, long long M, long long N, int bits, int zeroThr)
+enum
 {
-    __shared__ double sv[DCHUNK];
+    DWALK_SUM = 0, // acc += v
+    DWALK_SQUARES, // acc += v * v
+    DWALK_BELOW,   // acc += v where v < threshold (every other row adds +0: the sum starts at +0 and stays exact)
+    DWALK_REST     // acc += v in all other rows (a NaN lands here, as in the reference)
+};
+template <int KIND>
+__device__ __forceinline__ double dwalk_term(double v, double threshold)
+{
+    if (KIND == DWALK_SQUARES)
+        return __dmul_rn(v, v);
+    if (KIND == DWALK_BELOW)
+        return (v < threshold) ? v : 0.0;
+    if (KIND == DWALK_REST)
+        return (v < threshold) ? 0.0 : v;
+    return v;
+}
+// one lane, rows in order; eight rows per trip with the next eight already loaded (the prefetch of the last trip is clamped)
+template <int KIND>
+__device__ __forceinline__ double dwalk(const double* __restrict__ sv, int nr, double acc, double threshold)
+{
+    const int trips = nr >> 3;
+    const double2* const p = reinterpret_cast<const double2*>(sv);
+    if (trips > 0)
+    {
+        double2 a[4], n[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            a[i] = p[i];
+        for (int t = 0; t < trips; ++t)
+        {
+            const int nx = (t + 1 < trips ? t + 1 : t) * 4;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                n[i] = p[nx + i];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+            {
+                acc = __dadd_rn(acc, dwalk_term<KIND>(a[i].x, threshold));
+                acc = __dadd_rn(acc, dwalk_term<KIND>(a[i].y, threshold));
+                a[i] = n[i];
+            }
+        }
+    }
+    for (int i = trips << 3; i < nr; ++i)
+        acc = __dadd_rn(acc, dwalk_term<KIND>(sv[i], threshold));
+    return acc;
+}
+
+// stages rows [r0, r0 + nr) of v = gradient + residual and returns how many of this thread's rows are below `threshold`
+__device__ __forceinline__ unsigned dstage(double* __restrict__ sv, const double* __restrict__ g, const double* r, int nr, double threshold)
+{
+    unsigned below = 0;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < nr; i += blockDim.x)
+    {
+        const double v = __dadd_rn(g[i], r[i]);
+        sv[i] = v;
+        below += (v < threshold) ? 1u : 0u;
+    }
+    return below;
+}
+
+// ComputeRangeStatColjSubset for one column (ColumnQuantizer.h:209-341) + Quantize (ColumnQuantizer.h:50-65, 90-147).
+// `chunk` rows are staged at a time; a column of up to `chunk` rows is read from memory once and stays for the quantization.
+__global__ void __launch_bounds__(256) k_quantize_f64(const double* __restrict__ grad, const double* resIn, double* resOut,
+                                                     unsigned char* __restrict__ packed, long long M, long long N, int bits, int zeroThr, int chunk)
+{
+    extern __shared__ __align__(16) double sv[];
+    __shared__ unsigned long long sWords[DWORDS];
     __shared__ double sAcc[2];
     __shared__ unsigned sNum0;
     __shared__ double sRange[2];
-    const int tid = threadIdx.x;
-    const long long Q = (M * bits + 63) / 64;
-    const long long colBytes = 16 + 8 * Q;
+    const int tid = threadIdx.x, nt = blockDim.x;
+    const int Q = (int) ((M * bits + 63) / 64); // M < 2^30, so with 64 bits Q = M still fits
+    const long long colBytes = 16 + 8 * (long long) Q;
     const int vpw = 64 / bits;
+    const bool resident = M <= chunk;
+    // Threads per packed word.  Word w holds rows w, w + Q, ...: with few words (a 512-row column has 8 at 1 bit) one thread
+    // per word would leave the CTA idle, so `split` threads take every split-th row of a word and OR their fields together in
+    // shared memory; task t = (t / Q, t % Q) then covers rows t, t + split * Q, ...: neighbouring threads, neighbouring rows.
+    const int split = (Q > DWORDS / 2) ? 1 : min(vpw, DWORDS / Q);
+    const int tasks = Q * split; // split > 1: at most DWORDS
     for (long long j = blockIdx.x; j < N; j += gridDim.x)
     {
         const double* __restrict__ g = grad + j * M;
-        const double* __restrict__ r = resIn + j * M;
+        const double* r = resIn + j * M;
         const double rows = (double) (unsigned long long) M; // size_t -> double
         double mean = 0.0;
+        if (tid == 0)
+            sNum0 = 0u;
+        if (split > 1)
+            for (int w = tid; w < Q; w += nt)
+                sWords[w] = 0ull;
+        __syncthreads();
         // mean-threshold 1-bit mode: a first ordered pass for the column mean (:232-245)
         if (bits == 1 && !zeroThr)
         {
             double acc = 0.0;
-            for (long long r0 = 0; r0 < M; r0 += DCHUNK)
+            for (long long r0 = 0; r0 < M; r0 += chunk)
             {
-                const int nr = (int) min((long long) DCHUNK, M - r0);
-                for (int i = tid; i < nr; i += DNT)
-                    sv[i] = __dadd_rn(g[r0 + i], r[r0 + i]);
+                const int nr = (int) min((long long) chunk, M - r0);
+                dstage(sv, g + r0, r + r0, nr, 0.0);
                 __syncthreads();
                 if (tid == 0)
-                    for (int i = 0; i < nr; ++i)
-                        acc = __dadd_rn(acc, sv[i]);
+                    acc = dwalk<DWALK_SUM>(sv, nr, acc, 0.0);
                 __syncthreads();
             }
             if (tid == 0)
                 sAcc[0] = __ddiv_rn(acc, rows);
             __syncthreads();
             mean = sAcc[0];
-            __syncthreads();
         }
         // the ordered sums: two level sums and a count (1 bit), or the sum of squares (otherwise)
         double acc = 0.0;
-        unsigned num0 = 0;
-        for (long long r0 = 0; r0 < M; r0 += DCHUNK)
+        for (long long r0 = 0; r0 < M; r0 += chunk)
         {
-            const int nr = (int) min((long long) DCHUNK, M - r0);
-            for (int i = tid; i < nr; i += DNT)
-                sv[i] = __dadd_rn(g[r0 + i], r[r0 + i]);
+            const int nr = (int) min((long long) chunk, M - r0);
+            unsigned below = 0;
+            if (resident && bits == 1 && !zeroThr) // already staged
+                for (int i = tid; i < nr; i += nt)
+                    below += (sv[i] < mean) ? 1u : 0u;
+            else
+                below = dstage(sv, g + r0, r + r0, nr, mean);
+            if (bits == 1)
+            {
+                below = __reduce_add_sync(0xffffffffu, below);
+                if ((tid & 31) == 0 && below)
+                    atomicAdd(&sNum0, below);
+            }
             __syncthreads();
             if (bits == 1)
             {
-                if (tid == 0) // lower level: the rows with v < mean, counted; every other row adds +0 (the sum starts at +0 and stays exact)
-                    for (int i = 0; i < nr; ++i)
-                    {
-                        const double v = sv[i];
-                        const bool below = v < mean;
-                        acc = __dadd_rn(acc, below ? v : 0.0);
-                        num0 += below ? 1u : 0u;
-                    }
-                else if (tid == 32) // upper level: all other rows (a NaN lands here, as in the reference)
-                    for (int i = 0; i < nr; ++i)
-                    {
-                        const double v = sv[i];
-                        acc = __dadd_rn(acc, (v < mean) ? 0.0 : v);
-                    }
+                if (tid == 0)
+                    acc = dwalk<DWALK_BELOW>(sv, nr, acc, mean);
+                else if (tid == 32)
+                    acc = dwalk<DWALK_REST>(sv, nr, acc, mean);
             }
             else if (tid == 0)
             {
-                for (int i = 0; i < nr; ++i)
-                {
-                    const double d = __dsub_rn(sv[i], mean);
-                    acc = __dadd_rn(acc, __dmul_rn(d, d));
-                }
+                acc = dwalk<DWALK_SQUARES>(sv, nr, acc, 0.0);
             }
-            __syncthreads();
-        }
-        if (tid == 0)
-        {
-            sAcc[0] = acc;
-            sNum0 = num0;
+            if (!resident)
+                __syncthreads();
         }
         if (tid == 32)
             sAcc[1] = acc;
@@ -158,7 +226,7 @@ __global__ void __launch_bounds__(DNT) k_quantize_f64(const double* __restrict__
             if (bits == 1)
             {
                 unsigned n0 = sNum0, n1 = (unsigned) M - sNum0;
-                const double a0 = sAcc[0], a1 = sAcc[1];
+                const double a0 = acc, a1 = sAcc[1];
                 double radius, newmean;
                 if (!zeroThr)
                 {
@@ -184,7 +252,7 @@ __global__ void __launch_bounds__(DNT) k_quantize_f64(const double* __restrict__
             }
             else
             {
-                const double stddev = __dsqrt_rn(__ddiv_rn(sAcc[0], rows));
+                const double stddev = __dsqrt_rn(__ddiv_rn(acc, rows));
                 const double w = __dmul_rn((double) 4.0f, stddev);
                 lower = __dsub_rn(mean, w);
                 upper = __dadd_rn(mean, w);
@@ -196,50 +264,75 @@ __global__ void __launch_bounds__(DNT) k_quantize_f64(const double* __restrict__
             hdr[1] = upper;
         }
         __syncthreads();
-        // QuantizeOneQWord: thread <-> packed word w, rows w, w + Q, ...
+        // QuantizeOneQWord
         const ValQD q = make_valq_d(bits, sRange[0], sRange[1]);
+        const double level0 = unquantize_d(q, bits, 0ull), level1 = unquantize_d(q, bits, 1ull); // 1 bit
         unsigned long long* __restrict__ words = reinterpret_cast<unsigned long long*>(packed + j * colBytes + 16);
-        double* __restrict__ ro = resOut + j * M;
-        for (long long w = tid; w < Q; w += DNT)
+        double* ro = resOut + j * M;
+        for (int t = tid; t < tasks; t += nt)
         {
+            const int part = t / Q, w = t - part * Q;
             unsigned long long word = 0ull;
-            long long i = w;
-            for (int k = 0; k < vpw && i < M; ++k, i += Q)
+            long long i = t; // = w + part * Q
+            for (int k = part; k < vpw && i < M; k += split, i += tasks)
             {
-                const double v = __dadd_rn(g[i], r[i]);
+                const double v = resident ? sv[i] : __dadd_rn(g[i], r[i]);
                 const unsigned long long qv = quantize_d(q, bits, zeroThr != 0, v);
-                ro[i] = __dsub_rn(v, unquantize_d(q, bits, qv));
+                ro[i] = __dsub_rn(v, bits == 1 ? (qv ? level1 : level0) : unquantize_d(q, bits, qv));
                 word |= qv << (k * bits);
             }
-            words[w] = word;
+            if (split == 1)
+                words[w] = word;
+            else if (word)
+                atomicOr(&sWords[w], word);
         }
         __syncthreads();
+        if (split > 1)
+            for (int w = tid; w < Q; w += nt)
+                words[w] = sWords[w];
+        // the next column's first barrier comes before anything overwrites sv; its clearing of sWords touches the same words
+        // from the same threads
     }
 }
 
-// UnquantizeOneQWord (ColumnQuantizer.h:150-203): thread <-> packed word
+// UnquantizeOneQWord (ColumnQuantizer.h:150-203).  Unit = `unitRows` consecutive rows of one column = one warp: row i is field
+// i / Q of word i % Q, neighbouring lanes read neighbouring words and write neighbouring rows.  (One thread per packed word
+// instead gave a 512 x 363 matrix 2904 threads with 64 serial, scattered stores each.)
 __global__ void __launch_bounds__(256) k_unquantize_f64(const unsigned char* __restrict__ packed, double* __restrict__ out, long long M, long long N, int bits,
-                                                        int add)
+                                                        int add, int unitRows)
 {
-    const long long Q = (M * bits + 63) / 64;
-    const long long colBytes = 16 + 8 * Q;
-    const int vpw = 64 / bits;
-    const long long total = N * Q;
-    for (long long t = (long long) blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long) gridDim.x * blockDim.x)
+    const unsigned Q = (unsigned) ((M * bits + 63) / 64);
+    const long long colBytes = 16 + 8 * (long long) Q;
+    const long long perCol = (M + unitRows - 1) / unitRows;
+    const long long total = N * perCol;
+    const unsigned lane = threadIdx.x & 31;
+    const unsigned advK = 32u / Q, advW = 32u - advK * Q;
+    for (long long t = ((long long) blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < total; t += ((long long) gridDim.x * blockDim.x) >> 5)
     {
-        const long long j = t / Q, w = t - j * Q;
+        const long long j = t / perCol;
+        const unsigned r0 = (unsigned) (t - j * perCol) * (unsigned) unitRows;
+        const unsigned end = (unsigned) min((long long) r0 + unitRows, M);
         const unsigned char* colp = packed + j * colBytes;
         const ValQD q = make_valq_d(bits, reinterpret_cast<const double*>(colp)[0], reinterpret_cast<const double*>(colp)[1]);
-        const unsigned long long word = reinterpret_cast<const unsigned long long*>(colp + 16)[w];
+        const unsigned long long* __restrict__ words = reinterpret_cast<const unsigned long long*>(colp + 16);
         const unsigned long long mask = q.rangeend - 1ull; // all ones when rangeend == 0 (full-word pass-through)
         double* __restrict__ o = out + j * M;
-        long long i = w;
-        for (int k = 0; k < vpw && i < M; ++k, i += Q)
+        unsigned i = r0 + lane;
+        unsigned k = i / Q, w = i - k * Q;
+#pragma unroll 4
+        for (; i < end; i += 32u)
         {
-            double v = unquantize_d(q, bits, (word >> (k * bits)) & mask);
+            double v = unquantize_d(q, bits, (words[w] >> (k * (unsigned) bits)) & mask);
             if (add)
                 v = __dadd_rn(v, o[i]);
             o[i] = v;
+            w += advW;
+            k += advK;
+            if (w >= Q)
+            {
+                w -= Q;
+                ++k;
+            }
         }
     }
 }
@@ -284,7 +377,19 @@ int qagg_quantize_f64(void* stream, const double* grad, const double* res_in, do
         (reinterpret_cast<uintptr_t>(res_out) & 7))
         return fail(QAGG_EINVAL, "qagg_quantize_f64: buffers must be 8-byte aligned");
     const int grid = (int) (N < 148 * 16 ? N : 148 * 16);
-    k_quantize_f64<<<grid, DNT, 0, (cudaStream_t) stream>>>(grad, res_in, res_out, static_cast<unsigned char*>(packed), M, N, bits, zero_threshold ? 1 : 0);
+    const int chunk = M <= DRESIDENT ? (int) M : DCHUNK;
+    const size_t smem = ((size_t) chunk * sizeof(double) + 15) & ~(size_t) 15;
+    if (smem > 32 * 1024) // with the kernel's static arrays this passes the 48 KB that need no attribute
+    {
+        const int rc = check_cuda(cudaFuncSetAttribute(k_quantize_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, DRESIDENT * (int) sizeof(double)),
+                                  "double quantize kernel attribute");
+        if (rc)
+            return rc;
+    }
+    // a short column cannot feed eight warps; with four, twice as many columns are in flight per SM
+    const int threads = M <= 512 ? 128 : 256;
+    k_quantize_f64<<<grid, threads, smem, (cudaStream_t) stream>>>(grad, res_in, res_out, static_cast<unsigned char*>(packed), M, N, bits,
+                                                                   zero_threshold ? 1 : 0, chunk);
     return check_cuda(cudaGetLastError(), "double quantize kernel launch");
 }
 
@@ -300,11 +405,11 @@ int qagg_unquantize_f64(void* stream, const void* packed, double* out, int64_t M
         return fail(QAGG_EINVAL, "qagg_unquantize_f64: null pointer");
     if ((reinterpret_cast<uintptr_t>(packed) & 7) || (reinterpret_cast<uintptr_t>(out) & 7))
         return fail(QAGG_EINVAL, "qagg_unquantize_f64: buffers must be 8-byte aligned");
-    const long long total = N * ((M * bits + 63) / 64);
-    long long grid = (total + 255) / 256;
-    if (grid > 148 * 8)
-        grid = 148 * 8;
-    k_unquantize_f64<<<(int) grid, 256, 0, (cudaStream_t) stream>>>(static_cast<const unsigned char*>(packed), out, M, N, bits, add ? 1 : 0);
+    // 128 rows per warp while that leaves warps to spare on the chip, else 512 (fewer range divisions per value)
+    const int unitRows = N * ((M + 127) / 128) <= 148LL * 64 ? 128 : 512;
+    const long long total = N * ((M + unitRows - 1) / unitRows);
+    const long long grid = std::min<long long>((total + 7) / 8, 148 * 64);
+    k_unquantize_f64<<<(int) grid, 256, 0, (cudaStream_t) stream>>>(static_cast<const unsigned char*>(packed), out, M, N, bits, add ? 1 : 0, unitRows);
     return check_cuda(cudaGetLastError(), "double unquantize kernel launch");
 }
 

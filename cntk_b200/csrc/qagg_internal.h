@@ -140,7 +140,8 @@ int cols_per_item(long long M, long long N, int smemFloats, bool* resident, int 
 // (both re-zeroed by the kernel before it ends), [8 + smid] per-SM tickets that spread the walking warps.
 cudaError_t launch_colquant(cudaStream_t st, bool stripes, int mode, const QTensor* single, const QTensor* tensors,
                             const QItem* items, int nItems, int colsPerItem, const LaunchCfg& cfg, unsigned* counters = nullptr,
-                            const Signal* signal = nullptr);
+                            const Signal* signal = nullptr, bool expand = false);
+// (expand, here and in launch_stream1: dense tables only; every entry's `out` receives the unquantized matrix as well)
 // copies `bytes` (rounded up to 16) from local `src` to the same offset of every signal.bcastBase[], then releases signal.flag[]
 cudaError_t launch_push(cudaStream_t st, const void* src, size_t bytes, const Signal& signal, unsigned* counters, int numSMs);
 // one warp polls flags[i] (i < n, i != skip) until each is >= value (wrap-safe) or maxPolls polls have passed; on
@@ -199,7 +200,7 @@ bool encode_map_2d(void* out128, const float* base, long long M, long long N, in
 // always table-driven with a work queue (`counters` as for launch_colquant, required).  The kernel's waits for copies in
 // flight are bounded: if one runs out, bit 1 of *status is set and the kernel ends normally (results invalid)
 cudaError_t launch_stream1(cudaStream_t st, const QTensor* tensors, const QItem* items, int nItems, const LaunchCfg& cfg, unsigned* counters,
-                           const Signal* signal = nullptr, unsigned* status = nullptr);
+                           const Signal* signal = nullptr, unsigned* status = nullptr, bool expand = false);
 
 // ---- the owner's reduce-requantize for 1 bit with threshold 0, two kernels (qagg_owner.cu) -------------------------------
 // Table entries describe the owned stripes: src[] / nsrc / selfRaw / grad (raw own stripe), res_in == res_out (stripe

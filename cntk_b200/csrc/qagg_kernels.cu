@@ -403,29 +403,34 @@ __device__ __forceinline__ void walk_resident(const QTensor& T, int nc, int stri
 // =================================================================================================================
 // Phase C: quantize, pack, residual (QuantizeOneQWord, ColumnQuantizer.h:90-147).
 // =================================================================================================================
+// `val` receives what the packed field unquantizes to, `res` the residual.
 template <int MODE>
-__device__ __forceinline__ unsigned quant_one(const ValQ& q, int bits, float val0, float val1, float v, float& res)
+__device__ __forceinline__ unsigned quant_one(const ValQ& q, int bits, float val0, float val1, float v, float& res, float& val)
 {
     if (MODE == MODE_MULTIBIT)
     {
         const unsigned qv = quantize_multibit(q, bits, v);
-        res = __fsub_rn(v, unquantize_val(q, bits, qv));
+        val = unquantize_val(q, bits, qv);
+        res = __fsub_rn(v, val);
         return qv;
     }
     const bool bit = (MODE == MODE_ONEBIT_ZERO) ? (v >= 0.0f) : (v >= q.qmid);
-    res = __fsub_rn(v, bit ? val1 : val0);
+    val = bit ? val1 : val0;
+    res = __fsub_rn(v, val);
     return bit ? 1u : 0u;
 }
 
 template <int MODE>
 __device__ __forceinline__ void quantize_resident(const QTensor& T, const Signal& sg, int col0, int nc, int stride, const float* __restrict__ smem,
-                                                  const ColStats& S)
+                                                  const ColStats& S, bool expand)
 {
     const int M = (int) T.M;
     const int Q = T.Q;
     const int bits = T.bits;
     const int vpw = 32 / bits;
-    const bool vec = ((Q & 3) == 0) && ((M & 3) == 0) && ((reinterpret_cast<uintptr_t>(T.res_out) & 15) == 0);
+    float* const outBase = expand ? T.out : nullptr;
+    const bool vec = ((Q & 3) == 0) && ((M & 3) == 0) && ((reinterpret_cast<uintptr_t>(T.res_out) & 15) == 0) &&
+                     ((reinterpret_cast<uintptr_t>(outBase) & 15) == 0);
     if (vec)
     {
         // thread <-> four adjacent words: rows 4*w4 + k*Q .. +3 are one float4 in shared and in global memory
@@ -448,19 +453,22 @@ __device__ __forceinline__ void quantize_resident(const QTensor& T, const Signal
             }
             const float* __restrict__ vp = smem + (size_t) col * stride + w;
             float* __restrict__ rp = T.res_out + (size_t) j * M + w;
+            float* const op = outBase + (size_t) j * M + w;
             const int nk = min(vpw, (M - w + Q - 1) / Q);
             unsigned w0 = 0, w1 = 0, w2 = 0, w3 = 0;
 #pragma unroll 4
             for (int k = 0; k < nk; ++k)
             {
                 const float4 v = *reinterpret_cast<const float4*>(vp + k * Q);
-                float4 r;
+                float4 r, x;
                 const int sh = k * bits;
-                w0 |= quant_one<MODE>(q, bits, val0, val1, v.x, r.x) << sh;
-                w1 |= quant_one<MODE>(q, bits, val0, val1, v.y, r.y) << sh;
-                w2 |= quant_one<MODE>(q, bits, val0, val1, v.z, r.z) << sh;
-                w3 |= quant_one<MODE>(q, bits, val0, val1, v.w, r.w) << sh;
+                w0 |= quant_one<MODE>(q, bits, val0, val1, v.x, r.x, x.x) << sh;
+                w1 |= quant_one<MODE>(q, bits, val0, val1, v.y, r.y, x.y) << sh;
+                w2 |= quant_one<MODE>(q, bits, val0, val1, v.z, r.z, x.z) << sh;
+                w3 |= quant_one<MODE>(q, bits, val0, val1, v.w, r.w, x.w) << sh;
                 __stcs(reinterpret_cast<float4*>(rp + k * Q), r);
+                if (outBase)
+                    __stcs(reinterpret_cast<float4*>(op + k * Q), x);
             }
             const unsigned ws[4] = {w0, w1, w2, w3};
             store_words(T, sg, j, w, ws, 4, lower, upper);
@@ -486,14 +494,17 @@ __device__ __forceinline__ void quantize_resident(const QTensor& T, const Signal
             }
             const float* __restrict__ vp = smem + (size_t) col * stride + w;
             float* __restrict__ rp = T.res_out + (size_t) j * M + w;
+            float* const op = outBase + (size_t) j * M + w;
             const int nk = min(vpw, (M - w + Q - 1) / Q);
             unsigned word = 0;
 #pragma unroll 8
             for (int k = 0; k < nk; ++k)
             {
-                float r;
-                word |= quant_one<MODE>(q, bits, val0, val1, vp[k * Q], r) << (k * bits);
+                float r, x;
+                word |= quant_one<MODE>(q, bits, val0, val1, vp[k * Q], r, x) << (k * bits);
                 rp[k * Q] = r;
+                if (outBase)
+                    op[k * Q] = x;
             }
             store_words(T, sg, j, w, &word, 1, lower, upper);
         }
@@ -502,7 +513,7 @@ __device__ __forceinline__ void quantize_resident(const QTensor& T, const Signal
 
 // same, for streamed columns: the values are recomputed from the inputs
 template <int MODE, bool STRIPES>
-__device__ __forceinline__ void quantize_streamed(const QTensor& T, const Signal& sg, int col0, int nc, const ColStats& S)
+__device__ __forceinline__ void quantize_streamed(const QTensor& T, const Signal& sg, int col0, int nc, const ColStats& S, bool expand)
 {
     const int M = (int) T.M;
     const int Q = T.Q;
@@ -517,14 +528,17 @@ __device__ __forceinline__ void quantize_streamed(const QTensor& T, const Signal
         const float lower = S.lower[col], upper = S.upper[col];
         const ValQ q = make_valq(bits, lower, upper);
         const float val0 = unquantize_val(q, 1, 0u), val1 = unquantize_val(q, 1, 1u);
-        float* __restrict__ rp = T.res_out + (size_t) j * M + w;
+        float* rp = T.res_out + (size_t) j * M + w;
+        float* op = expand ? T.out + (size_t) j * M + w : nullptr;
         const int nk = min(vpw, (M - w + Q - 1) / Q);
         unsigned word = 0;
         for (int k = 0; k < nk; ++k)
         {
-            float r;
-            word |= quant_one<MODE>(q, bits, val0, val1, load_v<STRIPES>(T, j, (long long) w + (long long) k * Q), r) << (k * bits);
+            float r, x;
+            word |= quant_one<MODE>(q, bits, val0, val1, load_v<STRIPES>(T, j, (long long) w + (long long) k * Q), r, x) << (k * bits);
             rp[(size_t) k * Q] = r;
+            if (op)
+                op[(size_t) k * Q] = x;
         }
         store_words(T, sg, j, w, &word, 1, lower, upper);
     }
@@ -535,6 +549,9 @@ __device__ __forceinline__ void quantize_streamed(const QTensor& T, const Signal
 //   A. all threads stage the columns' fp32 values in shared memory (one coalesced pass over the inputs);
 //   B. the columns are walked in row order and each column's range is derived;
 //   C. all threads quantize, pack words, write the residual and the packed column to its owner's buffer.
+// `expand` (one rank: nothing is added to what this rank quantized): phase C also stores what each field unquantizes to into
+// T.out, which may be the gradient itself (a column's inputs are read before its phase C, by the same CTA), and no
+// unquantize launch follows.  The kernel waits for add chains, not for memory, so the extra 4 bytes per value ride along.
 // Several CTAs are resident per SM, so one CTA's walk overlaps the others' memory phases.  Work items are
 // handed out through a global counter (tallest columns first) when `counters` is given.
 // Columns too tall to stage are streamed through shared memory in chunks for B and re-read for C.
@@ -545,7 +562,7 @@ template <bool STRIPES, int MODE, bool TABLE>
 #endif
 __global__ void __launch_bounds__(NT, QAGG_CTAS_PER_SM) k_colquant(const QTensor single, const QTensor* __restrict__ tensors,
                                                     const QItem* __restrict__ items, int nItems, int colsPerItem, int smemFloats,
-                                                    int numSMs, unsigned* __restrict__ counters, const Signal signal)
+                                                    int numSMs, unsigned* __restrict__ counters, const Signal signal, int expand)
 {
     extern __shared__ __align__(16) float smem[];
     __shared__ QTensor sT;
@@ -648,7 +665,7 @@ __global__ void __launch_bounds__(NT, QAGG_CTAS_PER_SM) k_colquant(const QTensor
                 }
                 __syncthreads();
             }
-            quantize_resident<MODE>(T, signal, col0, nc, stride, smem, S);
+            quantize_resident<MODE>(T, signal, col0, nc, stride, smem, S, TABLE && !STRIPES && expand);
         }
         else
         {
@@ -699,7 +716,7 @@ __global__ void __launch_bounds__(NT, QAGG_CTAS_PER_SM) k_colquant(const QTensor
                 S.upper[lane] = up;
             }
             __syncthreads();
-            quantize_streamed<MODE, STRIPES>(T, signal, col0, nc, S);
+            quantize_streamed<MODE, STRIPES>(T, signal, col0, nc, S, TABLE && !STRIPES && expand);
         }
     }
     // The last CTA to leave re-arms the work counter for the next launch and, if asked to, tells the peers that every
@@ -782,7 +799,7 @@ int cols_per_item(long long M, long long N, int smemFloats, bool* resident, int 
 
 template <bool STRIPES, int MODE, bool TABLE>
 static cudaError_t launch_cq(cudaStream_t st, const QTensor* single, const QTensor* tensors, const QItem* items,
-                             int nItems, int colsPerItem, const LaunchCfg& cfg, unsigned* counters, const Signal& signal)
+                             int nItems, int colsPerItem, const LaunchCfg& cfg, unsigned* counters, const Signal& signal, bool expand)
 {
     auto kern = k_colquant<STRIPES, MODE, TABLE>;
     const size_t smemBytes = (size_t) cfg.smemFloats * sizeof(float);
@@ -793,7 +810,7 @@ static cudaError_t launch_cq(cudaStream_t st, const QTensor* single, const QTens
     if (grid > nItems)
         grid = nItems;
     static const QTensor zero = {};
-    kern<<<grid, NT, smemBytes, st>>>(single ? *single : zero, tensors, items, nItems, colsPerItem, cfg.smemFloats, cfg.numSMs, counters, signal);
+    kern<<<grid, NT, smemBytes, st>>>(single ? *single : zero, tensors, items, nItems, colsPerItem, cfg.smemFloats, cfg.numSMs, counters, signal, expand ? 1 : 0);
     return cudaGetLastError();
 }
 
@@ -896,7 +913,7 @@ cudaError_t launch_wait_flags(cudaStream_t st, const unsigned* flags, int n, int
 }
 
 cudaError_t launch_colquant(cudaStream_t st, bool stripes, int mode, const QTensor* single, const QTensor* tensors,
-                            const QItem* items, int nItems, int colsPerItem, const LaunchCfg& cfg, unsigned* counters, const Signal* signalp)
+                            const QItem* items, int nItems, int colsPerItem, const LaunchCfg& cfg, unsigned* counters, const Signal* signalp, bool expand)
 {
     static const Signal none = {};
     const Signal& signal = signalp ? *signalp : none;
@@ -913,7 +930,7 @@ cudaError_t launch_colquant(cudaStream_t st, bool stripes, int mode, const QTens
     const bool table = (single == nullptr);
 #define QAGG_CASE(S, MD, TB) \
     if (stripes == S && mode == MD && table == TB) \
-        return launch_cq<S, MD, TB>(st, single, tensors, items, nItems, colsPerItem, cfg, counters, signal);
+        return launch_cq<S, MD, TB>(st, single, tensors, items, nItems, colsPerItem, cfg, counters, signal, expand);
     QAGG_CASE(false, MODE_ONEBIT_ZERO, false)
     QAGG_CASE(false, MODE_ONEBIT_MEAN, false)
     QAGG_CASE(false, MODE_MULTIBIT, false)

@@ -65,6 +65,74 @@ __device__ __forceinline__ int stream_geometry(const QTensor& T, int ncols)
     return (T.boxCols[1] > 0 && ncols <= T.boxCols[1]) ? 1 : 0;
 }
 
+// One rank only: the item's packed words, still in shared memory, are expanded into T.out on the spot (T.out may be the
+// gradient: every chunk of the item has been fetched by then, and no other item reads these columns), so no unquantize launch
+// follows and the packed matrix is not read back.  A thread takes four consecutive rows of a column -- field row / Q of words
+// row % Q .. + 3 -- and stores them as one 16-byte vector; threads are dealt to the item's rows column after column, so short
+// columns keep all threads busy.
+__device__ __forceinline__ void expand_item(const QTensor& T, int col0, int nc, int Q, bool vec, const unsigned* pkw, const float* lv0, const float* lv1)
+{
+    const unsigned M = (unsigned) T.M;
+    float* const out = T.out + (size_t) col0 * M;
+    const unsigned units = vec ? M >> 2 : M; // per column
+    const unsigned advC = NT / units, advU = NT - advC * units;
+    // row / Q = (row * magic) >> 32 exactly: the error of the rounded-up reciprocal is below row * Q / 2^32 < 1 / Q for the
+    // rows this kernel takes (row < 32 Q, Q <= QAGG_STREAM_PKWORDS: row * Q < 2^28)
+    const unsigned magic = 0xffffffffu / (unsigned) Q + 1u; // 0 for Q = 1, where the field is the row itself
+    unsigned c = threadIdx.x / units, u = threadIdx.x - c * units;
+#pragma unroll 2
+    while (c < (unsigned) nc)
+    {
+        const unsigned row = vec ? 4u * u : u;
+        unsigned k = (Q == 1) ? row : __umulhi(row, magic);
+        unsigned w = row - k * (unsigned) Q;
+        const unsigned* const words = pkw + c * (unsigned) Q;
+        const float v0 = lv0[c], v1 = lv1[c];
+        float* const p = out + (size_t) c * M + row;
+        if (vec)
+        {
+            unsigned b0, b1, b2, b3;
+            if ((Q & 3) == 0)
+            {
+                const uint4 w4 = *reinterpret_cast<const uint4*>(words + w);
+                b0 = w4.x >> k;
+                b1 = w4.y >> k;
+                b2 = w4.z >> k;
+                b3 = w4.w >> k;
+            }
+            else
+            {
+                auto next = [&]() {
+                    const unsigned b = words[w] >> k;
+                    if (++w == (unsigned) Q)
+                    {
+                        w = 0u;
+                        ++k;
+                    }
+                    return b;
+                };
+                b0 = next();
+                b1 = next();
+                b2 = next();
+                b3 = next();
+            }
+            __stcs(reinterpret_cast<float4*>(p), make_float4((b0 & 1u) ? v1 : v0, (b1 & 1u) ? v1 : v0, (b2 & 1u) ? v1 : v0, (b3 & 1u) ? v1 : v0));
+        }
+        else
+        {
+            *p = ((words[w] >> k) & 1u) ? v1 : v0;
+        }
+        u += advU;
+        c += advC;
+        if (u >= units)
+        {
+            u -= units;
+            ++c;
+        }
+    }
+}
+
+template <bool EXPAND>
 __global__ void __launch_bounds__(NT + 32, ST_CTAS_PER_SM) k_stream1(const QTensor* __restrict__ tensors, const QItem* __restrict__ items, int nItems,
                                                                      unsigned* __restrict__ counters, const Signal signal, unsigned* __restrict__ status)
 {
@@ -445,6 +513,7 @@ __global__ void __launch_bounds__(NT + 32, ST_CTAS_PER_SM) k_stream1(const QTens
                         sNan[pcol[u]] = 1u;
             }
             const int fnc = nc, fQ = Q, fcol0 = col0; // the finishing item's geometry
+            const bool fvec = vec;
             if (vec)
                 pos += (unsigned) nchunks;
             // the next item's geometry and previous reconstruction values are fetched before this item's last steps
@@ -471,6 +540,11 @@ __global__ void __launch_bounds__(NT + 32, ST_CTAS_PER_SM) k_stream1(const QTens
                 levels_1bit(lo, up, v0, v1);
                 T.lv[2 * (size_t) (fcol0 + tid)] = v0;
                 T.lv[2 * (size_t) (fcol0 + tid) + 1] = v1;
+                if (EXPAND)
+                {
+                    sLv0[tid] = v0; // the element warps are done with the previous values
+                    sLv1[tid] = v1;
+                }
             }
             consumer_sync();
             // packed columns to their owners (and to the broadcast copies): warp <-> column, lane <-> word
@@ -491,6 +565,8 @@ __global__ void __launch_bounds__(NT + 32, ST_CTAS_PER_SM) k_stream1(const QTens
                     }
                 }
             }
+            if (EXPAND)
+                expand_item(T, fcol0, fnc, fQ, fvec, pkw, sLv0, sLv1);
             consumer_sync(); // the item is done with its shared-memory state and with its descriptor buffer
             if (tid == 0)
                 mbar_arrive(&sMetaEmpty[itemNo % ST_DESC]);
@@ -710,7 +786,7 @@ void stream_set_maps(QTensor* t, unsigned char* hostMaps, unsigned char* devMaps
 }
 
 cudaError_t launch_stream1(cudaStream_t st, const QTensor* tensors, const QItem* items, int nItems, const LaunchCfg& cfg, unsigned* counters,
-                           const Signal* signalp, unsigned* status)
+                           const Signal* signalp, unsigned* status, bool expand)
 {
     static const Signal none = {};
     const Signal& signal = signalp ? *signalp : none;
@@ -721,10 +797,11 @@ cudaError_t launch_stream1(cudaStream_t st, const QTensor* tensors, const QItem*
     int grid = cfg.numSMs * ST_CTAS_PER_SM;
     if (grid > nItems)
         grid = nItems;
-    cudaError_t e = cudaFuncSetAttribute(k_stream1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) ST_SMEM_BYTES);
+    auto kern = expand ? k_stream1<true> : k_stream1<false>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) ST_SMEM_BYTES);
     if (e != cudaSuccess)
         return e;
-    k_stream1<<<grid, NT + 32, ST_SMEM_BYTES, st>>>(tensors, items, nItems, counters, signal, status);
+    kern<<<grid, NT + 32, ST_SMEM_BYTES, st>>>(tensors, items, nItems, counters, signal, status);
     return cudaGetLastError();
 }
 
