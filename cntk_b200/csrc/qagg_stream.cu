@@ -16,8 +16,8 @@
 //     tensor copy per input (cp.async.bulk.tensor through a tensor map of the matrix: box = R rows x nc columns; an
 //     mbarrier per ring slot counts the bytes), as far ahead as the input ring has free slots -- across item
 //     boundaries too, so the consumers never wait for a pipeline to refill;
-//   * six "element" warps form v = gradient + (prev - level(prev)), store v to global memory and to a padded tile for the walkers, and OR the bit (v >= 0) into the item's packed
-//     words, which live in shared memory until the item ends;
+//   * six "element" warps form v = gradient + (prev - level(prev)), store v to global memory and to a padded tile for the
+//     walkers, and collect the bits (v >= 0), which live in shared memory until the item ends;
 //   * two "walker" warps (one per level, lane = column) add min(v, 0) resp. max(v, 0) of the previous chunk to their
 //     running sums, in row order;
 //   * at the end the ranges and the new reconstruction values are derived and the packed columns go to their owners.
@@ -41,7 +41,7 @@ constexpr int ST_IN_FLOATS = ST_TILE_VALUES;           // input tile: dense box,
 constexpr int ST_V_FLOATS = ST_TILE_VALUES + 4 * QAGG_STREAM_CMAX; // walkers' tile: column stride R + 4
 constexpr int ST_CTAS_PER_SM = 3;
 constexpr int ST_IN_STAGES = 4; // input ring slots: one being formed, the others in flight
-constexpr size_t ST_SMEM_BYTES = (size_t) (2 * ST_IN_STAGES * ST_IN_FLOATS + 2 * ST_V_FLOATS + QAGG_STREAM_PKWORDS) * 4;
+constexpr size_t ST_SMEM_BYTES = (size_t) (2 * ST_IN_STAGES * ST_IN_FLOATS + 2 * ST_V_FLOATS + QAGG_STREAM_PKWORDS + QAGG_STREAM_CMAX) * 4;
 
 // rows per chunk for a tile geometry of `boxCols` columns: a multiple of 32 (so that the walkers' tile, whose column
 // stride is R + 4, spreads the 128-bit reads of neighbouring columns over distinct banks), at most 256 (tensor copy box)
@@ -65,62 +65,63 @@ __device__ __forceinline__ int stream_geometry(const QTensor& T, int ncols)
     return (T.boxCols[1] > 0 && ncols <= T.boxCols[1]) ? 1 : 0;
 }
 
-// One rank only: the item's packed words, still in shared memory, are expanded into T.out on the spot (T.out may be the
-// gradient: every chunk of the item has been fetched by then, and no other item reads these columns), so no unquantize launch
-// follows and the packed matrix is not read back.  A thread takes four consecutive rows of a column -- field row / Q of words
-// row % Q .. + 3 -- and stores them as one 16-byte vector; threads are dealt to the item's rows column after column, so short
-// columns keep all threads busy.
-__device__ __forceinline__ void expand_item(const QTensor& T, int col0, int nc, int Q, bool vec, const unsigned* pkw, const float* lv0, const float* lv1)
+// The result bits of an item live in shared memory until it ends, in one of two forms.  Where the item is only packed
+// (EXPAND off), each bit is OR-ed into its packed word as it is formed.  Where the item is expanded too, they are collected in
+// ROW ORDER -- bit r of a column's bitmap is row r, column stride Q + 1 words, zero past the last row -- and turned into the
+// packed layout (bit k of word w = row w + kQ) once, at the item's end: the expansion then finds the bits of four consecutive
+// rows in one word, whatever Q is.  Measured on the speech set, both ways: expanding from packed words 169 us, from the bitmap
+// 151 us; packing alone 131 us with atomics, 135 us through the bitmap (the byte stores wait for a shuffle, and the item's end
+// for the transposition).
+// Eight neighbouring element threads own 32 consecutive rows, so a chunk's bits go into the bitmap with one byte store per
+// eight rows.  pack_fetch + pack_words give word w0 + lane: lane k fetches the 32 bits from row k * Q + w0 on (the 32 rows that
+// are bit k of words w0 .. w0 + 31) and the warp transposes the 32 x 32 bits.
+__device__ __forceinline__ unsigned pack_fetch(const unsigned* __restrict__ bitmap, int Q, int w0, int lane)
+{
+    const unsigned off = (unsigned) lane * (unsigned) Q + (unsigned) w0; // < 32 Q: the second word below is at most word Q
+    return __funnelshift_r(bitmap[off >> 5], bitmap[(off >> 5) + 1u], off & 31u);
+}
+// (PACK_ILP independent blocks at a time: a transposition alone is a chain of five shuffles)
+constexpr int PACK_ILP = 4;
+__device__ __forceinline__ void pack_words(unsigned (&x)[PACK_ILP], int lane)
+{
+#pragma unroll
+    for (int j = 16; j >= 1; j >>= 1)
+    {
+        const unsigned m = (j == 16) ? 0x0000ffffu : (j == 8) ? 0x00ff00ffu : (j == 4) ? 0x0f0f0f0fu : (j == 2) ? 0x33333333u : 0x55555555u;
+#pragma unroll
+        for (int i = 0; i < PACK_ILP; ++i)
+        {
+            const unsigned y = __shfl_xor_sync(0xffffffffu, x[i], j);
+            x[i] = (lane & j) ? ((x[i] & ~m) | ((y >> j) & m)) : ((x[i] & m) | ((y & m) << j));
+        }
+    }
+}
+
+// One rank only: the item's bits, still in shared memory, are expanded into T.out on the spot (T.out may be the gradient:
+// every chunk of the item has been fetched by then, and no other item uses these columns), so no unquantize launch follows and
+// the packed matrix is not read back.  A thread takes four consecutive rows of a column and stores them as one 16-byte
+// vector; threads are dealt to the item's rows column after column, so short columns keep all threads busy.
+__device__ __forceinline__ void expand_item(const QTensor& T, int col0, int nc, int Q, bool vec, const unsigned* bitmap, const float* lv0, const float* lv1)
 {
     const unsigned M = (unsigned) T.M;
     float* const out = T.out + (size_t) col0 * M;
     const unsigned units = vec ? M >> 2 : M; // per column
     const unsigned advC = NT / units, advU = NT - advC * units;
-    // row / Q = (row * magic) >> 32 exactly: the error of the rounded-up reciprocal is below row * Q / 2^32 < 1 / Q for the
-    // rows this kernel takes (row < 32 Q, Q <= QAGG_STREAM_PKWORDS: row * Q < 2^28)
-    const unsigned magic = 0xffffffffu / (unsigned) Q + 1u; // 0 for Q = 1, where the field is the row itself
     unsigned c = threadIdx.x / units, u = threadIdx.x - c * units;
-#pragma unroll 2
+#pragma unroll 4
     while (c < (unsigned) nc)
     {
-        const unsigned row = vec ? 4u * u : u;
-        unsigned k = (Q == 1) ? row : __umulhi(row, magic);
-        unsigned w = row - k * (unsigned) Q;
-        const unsigned* const words = pkw + c * (unsigned) Q;
+        const unsigned* const bits = bitmap + c * (unsigned) (Q + 1);
         const float v0 = lv0[c], v1 = lv1[c];
-        float* const p = out + (size_t) c * M + row;
         if (vec)
         {
-            unsigned b0, b1, b2, b3;
-            if ((Q & 3) == 0)
-            {
-                const uint4 w4 = *reinterpret_cast<const uint4*>(words + w);
-                b0 = w4.x >> k;
-                b1 = w4.y >> k;
-                b2 = w4.z >> k;
-                b3 = w4.w >> k;
-            }
-            else
-            {
-                auto next = [&]() {
-                    const unsigned b = words[w] >> k;
-                    if (++w == (unsigned) Q)
-                    {
-                        w = 0u;
-                        ++k;
-                    }
-                    return b;
-                };
-                b0 = next();
-                b1 = next();
-                b2 = next();
-                b3 = next();
-            }
-            __stcs(reinterpret_cast<float4*>(p), make_float4((b0 & 1u) ? v1 : v0, (b1 & 1u) ? v1 : v0, (b2 & 1u) ? v1 : v0, (b3 & 1u) ? v1 : v0));
+            const unsigned b = bits[u >> 3] >> (4u * (u & 7u));
+            __stcs(reinterpret_cast<float4*>(out + (size_t) c * M) + u,
+                   make_float4((b & 1u) ? v1 : v0, (b & 2u) ? v1 : v0, (b & 4u) ? v1 : v0, (b & 8u) ? v1 : v0));
         }
         else
         {
-            *p = ((words[w] >> k) & 1u) ? v1 : v0;
+            out[(size_t) c * M + u] = ((bits[u >> 5] >> (u & 31u)) & 1u) ? v1 : v0;
         }
         u += advU;
         c += advC;
@@ -141,7 +142,7 @@ __global__ void __launch_bounds__(NT + 32, ST_CTAS_PER_SM) k_stream1(const QTens
     float* const inG = dsm;                                  // input ring: gradient boxes
     float* const inP = dsm + SIN * ST_IN_FLOATS;             // input ring: previous-state boxes
     float* const vt = dsm + 2 * SIN * ST_IN_FLOATS;          // the formed values of two chunks: one being walked, one being written
-    // the item's packed words (nc x Q)
+    // the item's result bits: packed words (nc x Q), or in row order (nc x (Q + 1) words, see pack_fetch)
     unsigned* const pkw = reinterpret_cast<unsigned*>(dsm + 2 * SIN * ST_IN_FLOATS + 2 * ST_V_FLOATS);
     // work items in flight: buffer (n % ST_DESC) holds the CTA's n-th item: its queue index (>= nItems: the queue is
     // empty), the item and its matrix descriptor
@@ -288,15 +289,16 @@ __global__ void __launch_bounds__(NT + 32, ST_CTAS_PER_SM) k_stream1(const QTens
         const float* gbase = nullptr;
         const float* pbase = nullptr;
         float* obase = nullptr;
-        unsigned advK = 0, advW = 0;
         unsigned pos = 0;                   // ring position of the item's chunk 0
         float lvReg0 = 0.0f, lvReg1 = 0.0f; // thread c < nc: the previous reconstruction values of column c, loaded ahead
-        // An element thread owns the same ST_U 16-byte positions (column, four rows) of every chunk.  Row i of a column is
-        // bit i / Q of packed word i % Q; the position's (word, bit) pair moves by a fixed step from chunk to chunk.
+        // An element thread owns the same ST_U 16-byte positions (column, four rows) of every chunk.
         bool pv[ST_U];
         int iofs[ST_U], vofs[ST_U], pcol[ST_U], prow[ST_U];
         size_t gofs[ST_U];
-        unsigned pw[ST_U], pk[ST_U], nanf[ST_U];
+        unsigned nanf[ST_U];
+        // packed form: row i of a column is bit i / Q of packed word i % Q; the position's (word, bit) pair moves by a fixed step
+        // from chunk to chunk
+        unsigned advK = 0, advW = 0, pw[ST_U], pk[ST_U];
 
         // wait for the CTA's n-th item to be described, and take it over unless the queue was empty
         auto adopt = [&](unsigned n) -> bool {
@@ -317,8 +319,11 @@ __global__ void __launch_bounds__(NT + 32, ST_CTAS_PER_SM) k_stream1(const QTens
             gbase = T.grad;
             pbase = T.res_in;
             obase = T.res_out;
-            advK = (unsigned) R / (unsigned) Q;
-            advW = (unsigned) R - advK * (unsigned) Q;
+            if (!EXPAND)
+            {
+                advK = (unsigned) R / (unsigned) Q;
+                advW = (unsigned) R - advK * (unsigned) Q;
+            }
             const int R4 = R >> 2;
 #pragma unroll
             for (int u = 0; u < ST_U; ++u)
@@ -332,8 +337,11 @@ __global__ void __launch_bounds__(NT + 32, ST_CTAS_PER_SM) k_stream1(const QTens
                 iofs[u] = c * R + r;       // in the dense input box
                 vofs[u] = c * (R + 4) + r; // in the walkers' tile
                 gofs[u] = (size_t) (col0 + c) * (size_t) M + (size_t) r;
-                pk[u] = (unsigned) r / (unsigned) Q;
-                pw[u] = (unsigned) r - pk[u] * (unsigned) Q;
+                if (!EXPAND)
+                {
+                    pk[u] = (unsigned) r / (unsigned) Q;
+                    pw[u] = (unsigned) r - pk[u] * (unsigned) Q;
+                }
                 nanf[u] = 0u;
             }
             if (tid < nc)
@@ -350,9 +358,10 @@ __global__ void __launch_bounds__(NT + 32, ST_CTAS_PER_SM) k_stream1(const QTens
         {
             const QTensor& T = *Tp;
             const int vstride = R + 4;
+            const int bstride = EXPAND ? Q + 1 : Q; // words per column of the result bits
 
             // ---- per-item state ----------------------------------------------------------------------------------------
-            for (int i = tid; i < nc * Q; i += NT)
+            for (int i = tid; i < nc * bstride; i += NT)
                 pkw[i] = 0u;
             if (tid < nc)
             {
@@ -367,6 +376,7 @@ __global__ void __launch_bounds__(NT + 32, ST_CTAS_PER_SM) k_stream1(const QTens
                 const int inOff = (int) ((pos + (unsigned) q) % SIN) * ST_IN_FLOATS;
                 float* const vtile = vt + (q & 1) * ST_V_FLOATS;
                 const int row0 = q * R;
+                unsigned bits = 0u; // EXPAND: byte u holds the four rows' bits of position u
 #pragma unroll
                 for (int u = 0; u < ST_U; ++u)
                 {
@@ -401,16 +411,24 @@ __global__ void __launch_bounds__(NT + 32, ST_CTAS_PER_SM) k_stream1(const QTens
                             }
                         }
                         const float lv0 = sLv0[c], lv1 = sLv1[c];
-                        // the usual case: the four rows are the same bit of four adjacent words
-                        const bool flat = (nv == 4) && (pw[u] + 3u < (unsigned) Q);
                         float v[4];
 #pragma unroll
                         for (int i = 0; i < 4; ++i)
                             v[i] = __fadd_rn(agg[i], deferred_residual(prev[i], lv0, lv1));
-                        unsigned* const myWords = pkw + c * Q;
-                        if (flat)
+                        if (EXPAND)
                         {
-                            unsigned* const wp = myWords + pw[u];
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+                                if (i < nv)
+                                {
+                                    nanf[u] |= (v[i] != v[i]) ? 1u : 0u;
+                                    bits |= (v[i] >= 0.0f) ? 1u << (8 * u + i) : 0u;
+                                }
+                        }
+                        else if (nv == 4 && pw[u] + 3u < (unsigned) Q)
+                        {
+                            // the usual case: the four rows are the same bit of four adjacent words
+                            unsigned* const wp = pkw + c * Q + pw[u];
                             const unsigned m = 1u << pk[u];
                             nanf[u] |= ((v[0] != v[0]) | (v[1] != v[1]) | (v[2] != v[2]) | (v[3] != v[3])) ? 1u : 0u;
 #pragma unroll
@@ -429,7 +447,7 @@ __global__ void __launch_bounds__(NT + 32, ST_CTAS_PER_SM) k_stream1(const QTens
                                 {
                                     nanf[u] |= (v[i] != v[i]) ? 1u : 0u;
                                     if (v[i] >= 0.0f)
-                                        atomicOr(myWords + (w - over * (unsigned) Q), 1u << (pk[u] + over));
+                                        atomicOr(pkw + c * Q + (w - over * (unsigned) Q), 1u << (pk[u] + over));
                                 }
                             }
                         }
@@ -448,13 +466,28 @@ __global__ void __launch_bounds__(NT + 32, ST_CTAS_PER_SM) k_stream1(const QTens
                                     gout[i] = v[i];
                         }
                     }
-                    // on to the next chunk's rows
-                    pw[u] += advW;
-                    pk[u] += advK;
-                    if (pw[u] >= (unsigned) Q)
+                    if (!EXPAND)
                     {
-                        pw[u] -= (unsigned) Q;
-                        ++pk[u];
+                        // on to the next chunk's rows
+                        pw[u] += advW;
+                        pk[u] += advK;
+                        if (pw[u] >= (unsigned) Q)
+                        {
+                            pw[u] -= (unsigned) Q;
+                            ++pk[u];
+                        }
+                    }
+                }
+                if (EXPAND)
+                {
+                    // two threads' rows make a byte; a chunk's first row is a multiple of 32, so the pair sits on one
+                    bits |= __shfl_down_sync(0xffffffffu, bits, 1) << 4;
+                    if (!(lane & 1))
+                    {
+#pragma unroll
+                        for (int u = 0; u < ST_U; ++u)
+                            if (pv[u] && row0 + prow[u] < M)
+                                reinterpret_cast<unsigned char*>(pkw + pcol[u] * bstride)[(row0 + prow[u]) >> 3] = (unsigned char) (bits >> (8 * u));
                     }
                 }
             };
@@ -512,7 +545,7 @@ __global__ void __launch_bounds__(NT + 32, ST_CTAS_PER_SM) k_stream1(const QTens
                     if (pv[u] && nanf[u])
                         sNan[pcol[u]] = 1u;
             }
-            const int fnc = nc, fQ = Q, fcol0 = col0; // the finishing item's geometry
+            const int fnc = nc, fQ = Q, fcol0 = col0, fstride = bstride; // the finishing item's geometry
             const bool fvec = vec;
             if (vec)
                 pos += (unsigned) nchunks;
@@ -524,7 +557,7 @@ __global__ void __launch_bounds__(NT + 32, ST_CTAS_PER_SM) k_stream1(const QTens
             {
                 unsigned ones = 0;
                 for (int w = lane; w < fQ; w += 32)
-                    ones += __popc(pkw[c * fQ + w]);
+                    ones += __popc(pkw[c * fstride + w]);
                 ones = __reduce_add_sync(0xffffffffu, ones);
                 if (lane == 0)
                     sN0[c] = (unsigned) T.M - ones;
@@ -547,8 +580,10 @@ __global__ void __launch_bounds__(NT + 32, ST_CTAS_PER_SM) k_stream1(const QTens
                 }
             }
             consumer_sync();
-            // packed columns to their owners (and to the broadcast copies): warp <-> column, lane <-> word
+            // packed columns to their owners (and to the broadcast copies)
+            if (!EXPAND)
             {
+                // warp <-> column, lane <-> word
                 const int nb = T.bcast ? signal.nbcast : 0;
                 for (int c = warp; c < fnc; c += NWARPS)
                 {
@@ -562,6 +597,36 @@ __global__ void __launch_bounds__(NT + 32, ST_CTAS_PER_SM) k_stream1(const QTens
                             out[w] = pkw[c * fQ + w];
                         if (lane == 0)
                             store_header(d, sLower[c], sUpper[c]);
+                    }
+                }
+            }
+            else
+            {
+                // warp <-> 32 words of a column, lane <-> word (one rank: nobody to broadcast to)
+                const int blocks = (fQ + 31) >> 5;
+                const int tasks = fnc * blocks;
+                for (int t0 = warp; t0 < tasks; t0 += PACK_ILP * NWARPS)
+                {
+                    unsigned words[PACK_ILP];
+#pragma unroll
+                    for (int i = 0; i < PACK_ILP; ++i)
+                    {
+                        const int t = min(t0 + i * NWARPS, tasks - 1);
+                        const int c = t / blocks;
+                        words[i] = pack_fetch(pkw + c * fstride, fQ, 32 * (t - c * blocks), lane);
+                    }
+                    pack_words(words, lane);
+#pragma unroll
+                    for (int i = 0; i < PACK_ILP; ++i)
+                    {
+                        const int t = t0 + i * NWARPS;
+                        const int c = t / blocks;
+                        const int w = 32 * (t - c * blocks) + lane;
+                        if (t >= tasks || w >= fQ)
+                            continue;
+                        reinterpret_cast<unsigned*>(sDst[c] + 8)[w] = words[i];
+                        if (w == 0)
+                            store_header(sDst[c], sLower[c], sUpper[c]);
                     }
                 }
             }

@@ -305,6 +305,26 @@ def test_step_with_header_sums_it_in_rank_order(G, K, peer):
             c.destroy()
 
 
+# one rank: rows around a packed word, a bitmap byte, a chunk and a 32-word pack block; columns around an item's width;
+# rows that are no multiple of 4 take the plain loads and stores
+ONE_RANK_EDGES = [(1, 5), (3, 1), (4, 9), (31, 3), (32, 25), (33, 2), (36, 24), (127, 7), (128, 12), (132, 13), (252, 26), (260, 8),
+                  (1023, 5), (1024, 17), (1028, 11), (2052, 30), (4100, 9), (9308, 10)]
+
+
+@pytest.mark.parametrize("bits,zero_thr,tall_rows", [(1, True, None), (1, True, "1024"), (1, False, None), (4, True, None), (8, True, None)])
+def test_one_rank_expands_at_edges(G, oracle_port, bits, zero_thr, tall_rows, monkeypatch):
+    """One rank: the quantize kernel stores the unquantized values itself.  Gradients, residuals and packed words stay the
+    oracle's bits over three steps (every sum is taken in the oracle's order, so there is nothing to tolerate)."""
+    if tall_rows:
+        monkeypatch.setenv("QAGG_TALL_ROWS", tall_rows)  # form + walk + unquantize beside the streaming kernel
+
+    def inputs(K, step):
+        rng = np.random.default_rng(991 + step)
+        return [[(rng.standard_normal((N, M)) * 1e-2).astype(np.float32) for (M, N) in ONE_RANK_EDGES] for _ in range(K)]
+
+    run_group(G, oracle_port, ONE_RANK_EDGES, 1, bits, zero_thr, True, 3, inputs)
+
+
 @pytest.mark.parametrize("keep_plain", [False, True])
 def test_caller_owned_residual_buffers(G, oracle_port, keep_plain):
     """qagg_agg_bind_residuals: the error-feedback state lives in buffers the caller owns (the V2 interface's
