@@ -109,6 +109,14 @@ def test_edge_shapes_bit_exact(G, oracle_port, shape, bits, zero_thr):
         G.assert_same_bits(G.host(out_g), out_o, f"{shape} b{bits} it{it} output")
 
 
+# columns per item: the most that still leave an SM without one (dealt over 444 CTA slots) and one more (full items), single
+# columns, the 1024-value floor, columns streamed in chunks
+@pytest.mark.parametrize("shape", [(2052, 1176), (2052, 1177), (1001, 444), (1001, 445), (5, 4096), (1, 445), (1023, 9), (20000, 13)], ids=lambda s: f"{s[0]}x{s[1]}")
+@pytest.mark.parametrize("bits,zero_thr", [(1, True), (1, False), (4, True)])
+def test_dealt_columns_bit_exact(G, oracle_port, shape, bits, zero_thr):
+    test_edge_shapes_bit_exact(G, oracle_port, shape, bits, zero_thr)
+
+
 def test_separate_residual_buffers_and_unaligned_base(G, oracle_port):
     """inResidual != outResidual (the V2 communicator's use, QuantizedDistributedCommunicator.h:365) and a gradient
     that starts 4 bytes off a 16-byte boundary (scalar load path)."""
