@@ -88,6 +88,16 @@ def test_double_quantizer_bit_exact(env, M, N, bits, zero_thr):
         assert np.array_equal(out_c.view(np.uint64), out_g.view(np.uint64)), f"iteration {it}: output differs"
 
 
+# edges of the launch shapes: the tallest resident column and chunked ones (a remainder, none); as many columns as SM slots
+# (148 SMs x 5) and one more, which go in short chunks by four warps; columns of at most 64 rows by two; around the split of
+# words over threads and the pair of staging buffers; enough words for the word-per-thread unquantize kernel
+@pytest.mark.parametrize("M,N", [(24576, 2), (24577, 3), (28672, 2), (40001, 2), (1030, 740), (1030, 741), (1024, 800), (3073, 800), (64, 2400), (65, 2400),
+                                 (3, 9000), (512, 2400), (513, 800), (512, 6), (513, 6), (8192, 4), (8193, 4), (97, 33000), (200, 2000)])
+@pytest.mark.parametrize("bits,zero_thr", [(1, True), (1, False), (2, True), (16, True), (64, True)])
+def test_double_launch_shapes_bit_exact(env, M, N, bits, zero_thr):
+    test_double_quantizer_bit_exact(env, M, N, bits, zero_thr)
+
+
 def test_double_argument_errors(env):
     lib, _ = env
     t = torch.zeros(64, dtype=torch.float64, device="cuda")
@@ -135,7 +145,7 @@ def test_matrix_quantizer_impl_double_like_the_reference_unit_test(env, tmp_path
 def test_double_aggregator_bit_exact(env, K, bits, zero_thr, self_quant):
     """qagg_agg_f64_*: AllReduceDistGradAggregator<double> on an in-process group, four steps with the residuals carried:
     every rank's aggregate, residual and stripe residual byte-identical to the CPU restatement of the exchange run with
-    the double checker (includes tensors with fewer columns than ranks, single columns, a column taller than one chunk)."""
+    the double checker (includes tensors with fewer columns than ranks and single columns)."""
     lib, oracle = env
     from oracle import exchange as ox
     shapes = [(70, 9), (256, 33), (1500, 2), (64, 1), (5, 16)]
