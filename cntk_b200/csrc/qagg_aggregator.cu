@@ -353,6 +353,14 @@ int build_tables(qagg_aggregator* a)
     a->iK1.clear();
     a->iK2.clear();
     a->k2Units = 0;
+    // the tall matrices' tables, filled below while the residuals are deferred; bound residuals may end that (keep_plain)
+    a->hK1t.clear();
+    a->k1tTensor.clear();
+    a->k1tCol.clear();
+    a->iK1t.clear();
+    a->k1tUnits = 0;
+    a->hK3t.clear();
+    a->k3tUnits = 0;
     std::vector<std::pair<int64_t, QItem>> cost1, cost2;
     std::vector<std::pair<int64_t, int64_t>> shapes1, shapes2;
     for (int i = 0; i < T; ++i)
@@ -484,11 +492,6 @@ int build_tables(qagg_aggregator* a)
         long long tallRows = 16384;
         if (const char* e = std::getenv("QAGG_TALL_ROWS"))
             tallRows = std::atoll(e);
-        a->hK1t.clear();
-        a->k1tTensor.clear();
-        a->k1tCol.clear();
-        a->iK1t.clear();
-        a->k1tUnits = 0;
         std::vector<std::pair<long long, long long>> tallShapes;
         long long tallCols = 0;
         for (int i = 0; i < T; ++i)
@@ -518,8 +521,6 @@ int build_tables(qagg_aggregator* a)
                 tallCols += n;
             }
         }
-        a->hK3t.clear();
-        a->k3tUnits = 0;
         if (K == 1)
             for (int i : a->k1tTensor)
             {

@@ -325,6 +325,30 @@ def test_one_rank_expands_at_edges(G, oracle_port, bits, zero_thr, tall_rows, mo
     run_group(G, oracle_port, ONE_RANK_EDGES, 1, bits, zero_thr, True, 3, inputs)
 
 
+@pytest.mark.parametrize("shapes,plain,updating", [([(256, 9)], 1, 2), ([(20000, 9)], 3, 3), ([(256, 9), (20000, 9)], 4, 4)])
+def test_one_rank_launches_per_step(G, shapes, plain, updating):
+    """A quantize launch that expands; form, walk and unquantize of a tall matrix, beside the streaming kernel if there are other
+    matrices; the unquantize-update launch while a learner step is bound; and one launch again once bound residual buffers
+    are kept plain, which takes the form + walk pair out of use."""
+    from cntk_b200 import lib
+    comm = lib.Comm.create(None, 0, 1, 0)
+    a = lib.Aggregator(comm, shapes, 1)
+    t = [torch.zeros((N, M), dtype=torch.float32, device=G.DEV) for (M, N) in shapes]
+    p = [x.data_ptr() for x in t]
+    try:
+        assert a.launches_per_step == plain
+        a.bind_update(p, p)
+        a.set_update(True, 0.1, 0.9, 0.1)
+        assert a.launches_per_step == updating
+        a.set_update(False)
+        assert a.launches_per_step == plain
+        a.bind_residuals(p, [0] * len(p), True)
+        assert a.launches_per_step == 1
+    finally:
+        a.destroy()
+        comm.destroy()
+
+
 @pytest.mark.parametrize("keep_plain", [False, True])
 def test_caller_owned_residual_buffers(G, oracle_port, keep_plain):
     """qagg_agg_bind_residuals: the error-feedback state lives in buffers the caller owns (the V2 interface's
