@@ -206,6 +206,7 @@ struct qagg_aggregator
     std::vector<QTensor> hK3t;
     long long k3tUnits = 0;
     QTensor* dK3t = nullptr;
+    bool gradsOverlap = false; // two of the bound gradient matrices share memory
     QTensor *dK1 = nullptr, *dK2 = nullptr, *dK3 = nullptr;
     QItem *dI1 = nullptr, *dI2 = nullptr;
     // consumer fusion: a copy of the unquantize table whose destinations are the caller's parameter and smoothed-gradient
@@ -223,6 +224,7 @@ struct qagg_aggregator
         std::vector<float*> grads;
         QTensor *dK1 = nullptr, *dK2 = nullptr, *dK3 = nullptr, *dK1t = nullptr, *dK3t = nullptr;
         QItem *dI1 = nullptr, *dI2 = nullptr, *dI1t = nullptr;
+        bool overlap = false;
     };
     Binding bindings[2];
     int curBinding = 0;
@@ -651,6 +653,20 @@ int upload_tables(qagg_aggregator* a, int slot)
     return QAGG_OK;
 }
 
+// whether any two matrices of a gradient array share memory: a parameter listed twice, or a view of another's columns
+bool grads_overlap(const qagg_aggregator* a, float* const* grads)
+{
+    std::vector<std::pair<uintptr_t, uintptr_t>> spans;
+    for (int i = 0; i < a->T; ++i)
+        if (a->M[i] * a->N[i] > 0)
+            spans.push_back({reinterpret_cast<uintptr_t>(grads[i]), reinterpret_cast<uintptr_t>(grads[i] + a->M[i] * a->N[i])});
+    std::sort(spans.begin(), spans.end());
+    for (size_t i = 1; i < spans.size(); ++i)
+        if (spans[i].first < spans[i - 1].second)
+            return true;
+    return false;
+}
+
 int bind_grads(qagg_aggregator* a, float* const* grads, cudaStream_t st)
 {
     for (int s = 0; s < 2; ++s)
@@ -670,6 +686,7 @@ int bind_grads(qagg_aggregator* a, float* const* grads, cudaStream_t st)
             a->dK1t = b.dK1t;
             a->dI1t = b.dI1t;
             a->dK3t = b.dK3t;
+            a->gradsOverlap = b.overlap;
             return QAGG_OK;
         }
     }
@@ -722,6 +739,7 @@ int bind_grads(qagg_aggregator* a, float* const* grads, cudaStream_t st)
     b.dK1t = a->dK1t;
     b.dI1t = a->dI1t;
     b.dK3t = a->dK3t;
+    b.overlap = a->gradsOverlap = a->comm->K == 1 && grads_overlap(a, grads);
     a->curBinding = slot;
     return QAGG_OK;
 }
@@ -760,10 +778,11 @@ Signal make_signal(const qagg_aggregator* a, bool gatherPhase)
 }
 // One rank: what it quantized is the aggregate, so the quantize kernel stores the unquantized values itself and the
 // unquantize launch, which would read every packed word back, is left out.  With the learner step bound the launch stays: it
-// is the kernel that applies the update.
+// is the kernel that applies the update.  So it does where matrices share memory: every matrix has to be read before any of
+// them is written.
 bool quantize_expands(const qagg_aggregator* a)
 {
-    return a->comm->K == 1 && !a->updating;
+    return a->comm->K == 1 && !a->updating && !a->gradsOverlap;
 }
 int launch_k1(qagg_aggregator* a, cudaStream_t st)
 {

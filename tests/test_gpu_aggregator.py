@@ -325,6 +325,44 @@ def test_one_rank_expands_at_edges(G, oracle_port, bits, zero_thr, tall_rows, mo
     run_group(G, oracle_port, ONE_RANK_EDGES, 1, bits, zero_thr, True, 3, inputs)
 
 
+@pytest.mark.parametrize("bits,zero_thr,tall_rows", [(1, True, None), (1, True, "1024"), (1, False, None), (4, True, None)])
+def test_one_rank_gradients_that_share_memory(G, oracle_port, bits, zero_thr, tall_rows, monkeypatch):
+    """A matrix listed twice, and a view of another's last columns: each is quantized from what its buffer held before the
+    step, so equal columns come out equal however often they are listed; a step with separate buffers between them is
+    unaffected.  Two steps on each array of pointers, residuals carried."""
+    from cntk_b200 import lib
+    if tall_rows:
+        monkeypatch.setenv("QAGG_TALL_ROWS", tall_rows)
+    M, N = 2052, 700
+    shapes = [(M, N), (96, 5), (M, N), (M, 250)]
+    comm = lib.Comm.create(None, 0, 1, 0)
+    a = lib.Aggregator(comm, shapes, bits, lib.SELF_QUANTIZED | (lib.ZERO_THRESHOLD if zero_thr else 0))
+    st = ox.ExchangeState(shapes, 1)
+    rng = np.random.default_rng(55 + bits)
+    shared = [torch.empty((n, m), dtype=torch.float32, device=G.DEV) for (m, n) in shapes[:2]]
+    apart = [torch.empty((n, m), dtype=torch.float32, device=G.DEV) for (m, n) in shapes]
+    views = [shared[0], shared[1], shared[0], shared[0][N - 250:]]
+    try:
+        for step in range(6):
+            bufs = apart if step in (2, 3) else views
+            w, b = [(rng.standard_normal((n, m)) * 1e-3).astype(np.float32) for (m, n) in shapes[:2]]
+            grads = [[w, b, w.copy(), w[N - 250:].copy()]]
+            for t, g in zip(bufs, grads[0]):
+                t.copy_(torch.from_numpy(g))
+            ox.aggregate_step(oracle_port, st, grads, bits, zero_thr, True)
+            a.step([t.data_ptr() for t in bufs])
+            torch.cuda.synchronize()
+            for i, t in enumerate(bufs):
+                G.assert_same_bits(G.host(t), grads[0][i], f"step {step} tensor {i}")
+                res = torch.empty(t.shape, dtype=torch.float32, device=G.DEV)
+                a.copy_residual(i, 0, res.data_ptr())
+                G.assert_same_bits(G.host(res), st.res[0][i], f"step {step} tensor {i} residual")
+        a.check()
+    finally:
+        a.destroy()
+        comm.destroy()
+
+
 @pytest.mark.parametrize("shapes,plain,updating", [([(256, 9)], 1, 2), ([(20000, 9)], 3, 3), ([(256, 9), (20000, 9)], 4, 4)])
 def test_one_rank_launches_per_step(G, shapes, plain, updating):
     """A quantize launch that expands; form, walk and unquantize of a tall matrix, beside the streaming kernel if there are other
