@@ -530,7 +530,10 @@ __device__ __forceinline__ void quantize_resident(const QTensor& T, const Signal
     }
 }
 
-// same, for streamed columns: the values are recomputed from the inputs
+// same, for streamed columns: the values are recomputed from the inputs.  The outputs may be the inputs' own buffers, so the
+// compiler keeps every load behind the stores before it; AHEAD rows of a word are therefore loaded before the first of them is
+// stored (39997 x 13 at 4 bits: 198 us per step, 223 one row at a time; 8 rows ahead measured the same at 4 bits, but the kernel
+// then spills and eight 1024 x 1024 at 4 bits, which never come here, went from 41.9 to 45.9 us).
 template <int MODE, bool STRIPES>
 __device__ __forceinline__ void quantize_streamed(const QTensor& T, const Signal& sg, int col0, int nc, const ColStats& S, bool expand)
 {
@@ -538,6 +541,7 @@ __device__ __forceinline__ void quantize_streamed(const QTensor& T, const Signal
     const int Q = T.Q;
     const int bits = T.bits;
     const int vpw = 32 / bits;
+    constexpr int AHEAD = 4;
     const long long total = (long long) nc * Q;
     for (long long t = threadIdx.x; t < total; t += NT)
     {
@@ -551,13 +555,24 @@ __device__ __forceinline__ void quantize_streamed(const QTensor& T, const Signal
         float* op = expand ? T.out + (size_t) j * M + w : nullptr;
         const int nk = min(vpw, (M - w + Q - 1) / Q);
         unsigned word = 0;
-        for (int k = 0; k < nk; ++k)
+        for (int k0 = 0; k0 < nk; k0 += AHEAD)
         {
-            float r, x;
-            word |= quant_one<MODE>(q, bits, val0, val1, load_v<STRIPES>(T, j, (long long) w + (long long) k * Q), r, x) << (k * bits);
-            rp[(size_t) k * Q] = r;
-            if (op)
-                op[(size_t) k * Q] = x;
+            float v[AHEAD];
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u)
+                v[u] = (k0 + u < nk) ? load_v<STRIPES>(T, j, (long long) w + (long long) (k0 + u) * Q) : 0.0f;
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u)
+            {
+                const int k = k0 + u;
+                if (k >= nk)
+                    break;
+                float r, x;
+                word |= quant_one<MODE>(q, bits, val0, val1, v[u], r, x) << (k * bits);
+                rp[(size_t) k * Q] = r;
+                if (op)
+                    op[(size_t) k * Q] = x;
+            }
         }
         store_words(T, sg, j, w, &word, 1, lower, upper);
     }

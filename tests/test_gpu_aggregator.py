@@ -309,20 +309,27 @@ def test_step_with_header_sums_it_in_rank_order(G, K, peer):
 # rows that are no multiple of 4 take the plain loads and stores
 ONE_RANK_EDGES = [(1, 5), (3, 1), (4, 9), (31, 3), (32, 25), (33, 2), (36, 24), (127, 7), (128, 12), (132, 13), (252, 26), (260, 8),
                   (1023, 5), (1024, 17), (1028, 11), (2052, 30), (4100, 9), (9308, 10)]
+# columns too tall to stay in shared memory (mean threshold, more bits), or walked by the streaming kernel with plain loads; an
+# item whose row-order bits need more words than its packed ones; remainders of the rows a thread loads ahead
+ONE_RANK_TALL = [(10240, 9), (20001, 9), (20004, 3), (40000, 3), (50002, 2), (81920, 1), (37, 11)]
 
 
-@pytest.mark.parametrize("bits,zero_thr,tall_rows", [(1, True, None), (1, True, "1024"), (1, False, None), (4, True, None), (8, True, None)])
+@pytest.mark.parametrize("bits,zero_thr,tall_rows", [(1, True, None), (1, True, "1024"), (1, True, "0"), (1, False, None), (2, True, None), (4, True, None),
+                                                     (8, True, None), (32, True, None)])
 def test_one_rank_expands_at_edges(G, oracle_port, bits, zero_thr, tall_rows, monkeypatch):
     """One rank: the quantize kernel stores the unquantized values itself.  Gradients, residuals and packed words stay the
     oracle's bits over three steps (every sum is taken in the oracle's order, so there is nothing to tolerate)."""
     if tall_rows:
         monkeypatch.setenv("QAGG_TALL_ROWS", tall_rows)  # form + walk + unquantize beside the streaming kernel
 
-    def inputs(K, step):
-        rng = np.random.default_rng(991 + step)
-        return [[(rng.standard_normal((N, M)) * 1e-2).astype(np.float32) for (M, N) in ONE_RANK_EDGES] for _ in range(K)]
+    def inputs(shapes):
+        def make(K, step):
+            rng = np.random.default_rng(991 + step)
+            return [[(rng.standard_normal((N, M)) * 1e-2).astype(np.float32) for (M, N) in shapes] for _ in range(K)]
+        return make
 
-    run_group(G, oracle_port, ONE_RANK_EDGES, 1, bits, zero_thr, True, 3, inputs)
+    for shapes in (ONE_RANK_EDGES, ONE_RANK_TALL):
+        run_group(G, oracle_port, shapes, 1, bits, zero_thr, True, 3, inputs(shapes))
 
 
 @pytest.mark.parametrize("bits,zero_thr,tall_rows", [(1, True, None), (1, True, "1024"), (1, False, None), (4, True, None)])
