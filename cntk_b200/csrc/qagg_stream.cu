@@ -105,7 +105,10 @@ __device__ __forceinline__ void expand_item(const QTensor& T, int col0, int nc, 
 {
     const unsigned M = (unsigned) T.M;
     float* const out = T.out + (size_t) col0 * M;
-    const unsigned units = vec ? M >> 2 : M; // per column
+    // A column that is not 16-byte aligned has up to three rows before its first boundary and up to three after its last: they are
+    // stored one by one, in up to six units after the quads (with one row per unit throughout, the last item of a 39997 x 13
+    // matrix kept its CTA 25 us longer).
+    const unsigned units = vec ? M >> 2 : (M >> 2) + 6u; // per column
     const unsigned advC = NT / units, advU = NT - advC * units;
     unsigned c = threadIdx.x / units, u = threadIdx.x - c * units;
 #pragma unroll 4
@@ -121,7 +124,22 @@ __device__ __forceinline__ void expand_item(const QTensor& T, int col0, int nc, 
         }
         else
         {
-            out[(size_t) c * M + u] = ((bits[u >> 5] >> (u & 31u)) & 1u) ? v1 : v0;
+            float* const o = out + (size_t) c * M;
+            const unsigned head = min(M, (4u - ((unsigned) (reinterpret_cast<uintptr_t>(o) >> 2) & 3u)) & 3u);
+            const unsigned quads = (M - head) >> 2;
+            if (u < quads)
+            {
+                const unsigned i = head + 4u * u; // the word after the last row's is zero, and there (stride Q + 1)
+                const unsigned b = __funnelshift_r(bits[i >> 5], bits[(i >> 5) + 1u], i & 31u);
+                __stcs(reinterpret_cast<float4*>(o + i), make_float4((b & 1u) ? v1 : v0, (b & 2u) ? v1 : v0, (b & 4u) ? v1 : v0, (b & 8u) ? v1 : v0));
+            }
+            else
+            {
+                const unsigned e = u - quads;
+                const unsigned i = e < head ? e : e + 4u * quads;
+                if (i < M)
+                    o[i] = ((bits[i >> 5] >> (i & 31u)) & 1u) ? v1 : v0;
+            }
         }
         u += advU;
         c += advC;

@@ -332,6 +332,36 @@ def test_one_rank_expands_at_edges(G, oracle_port, bits, zero_thr, tall_rows, mo
         run_group(G, oracle_port, shapes, 1, bits, zero_thr, True, 3, inputs(shapes))
 
 
+@pytest.mark.parametrize("offset", [1, 2, 3])
+@pytest.mark.parametrize("bits,zero_thr", [(1, True), (1, False), (4, True)])
+def test_one_rank_unaligned_gradients(G, oracle_port, bits, zero_thr, offset):
+    """Gradients that start 4, 8 or 12 bytes off a 16-byte boundary: every column's first and last rows are stored one by one,
+    also where a column has none between them, and nothing around the matrices is touched."""
+    from cntk_b200 import lib
+    shapes = [(256, 30), (1, 9), (2, 7), (3, 5), (4, 3), (5, 40), (6, 2), (7, 6), (8, 4), (33, 12), (2051, 9), (20001, 3), (20000, 2)]
+    comm = lib.Comm.create(None, 0, 1, 0)
+    a = lib.Aggregator(comm, shapes, bits, lib.SELF_QUANTIZED | (lib.ZERO_THRESHOLD if zero_thr else 0))
+    st = ox.ExchangeState(shapes, 1)
+    rng = np.random.default_rng(31 * bits + offset)
+    bufs = [torch.full((m * n + 12,), 7.0, dtype=torch.float32, device=G.DEV) for (m, n) in shapes]
+    views = [b[4 + offset:4 + offset + m * n].view(n, m) for b, (m, n) in zip(bufs, shapes)]
+    try:
+        for step in range(3):
+            grads = [[(rng.standard_normal((n, m)) * 1e-3).astype(np.float32) for (m, n) in shapes]]
+            for t, g in zip(views, grads[0]):
+                t.copy_(torch.from_numpy(g))
+            ox.aggregate_step(oracle_port, st, grads, bits, zero_thr, True)
+            a.step([t.data_ptr() for t in views])
+            torch.cuda.synchronize()
+            for i, (b, t) in enumerate(zip(bufs, views)):
+                G.assert_same_bits(G.host(t), grads[0][i], f"step {step} tensor {i}")
+                assert bool((b[:4 + offset] == 7.0).all()) and bool((b[4 + offset + t.numel():] == 7.0).all()), f"tensor {i}: stored outside the matrix"
+        a.check()
+    finally:
+        a.destroy()
+        comm.destroy()
+
+
 @pytest.mark.parametrize("bits,zero_thr,tall_rows", [(1, True, None), (1, True, "1024"), (1, False, None), (4, True, None)])
 def test_one_rank_gradients_that_share_memory(G, oracle_port, bits, zero_thr, tall_rows, monkeypatch):
     """A matrix listed twice, and a view of another's last columns: each is quantized from what its buffer held before the
