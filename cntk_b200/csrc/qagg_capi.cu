@@ -34,21 +34,34 @@ int mode_of(int bits, int zeroThr)
     return MODE_MULTIBIT;
 }
 
-// Columns per work item of a single-matrix launch, at most `fit`.  Items of as many columns as fit leave most of the chip idle
-// where the columns are short and few: a 1001 x 517 matrix made 29 items of 18 columns for 148 SMs.  Where that makes fewer
-// items than there are SMs, the columns are dealt evenly over the CTA slots (1001 x 517 with the mean threshold, quantize +
-// unquantize: 45.1 -> 25.0 us).  Once every SM has an item, full ones are the better: a CTA lasts as long as its column's add
-// chains anyway and with fewer columns has fewer copies in flight (2048 x 2048 in 410 items of 5 columns instead of 256 of
-// 8: 27.2 -> 28.7 us).  An item keeps 1024 values, four per thread.
-static int balanced_cols(long long M, long long N, int fit, const LaunchCfg& cfg)
+// Columns per work item of a single-matrix launch, at most as many as fit in shared memory.  The columns are dealt evenly
+// over two CTAs per SM.  Full items leave SMs idle where the columns are short and few (1001 x 517 made 29 items of 18); and a
+// third CTA on an SM puts a third walking warp on one scheduler, which the modes that walk two sums per column pay for.
+// More than one bit walks a single sum: there three CTAs are taken where they leave an SM fewer columns, or as many but with
+// plain loads, which are waited for longer.  Columns too tall to stay in shared memory take three: what they wait for is mostly
+// memory.  An item keeps 1024 values, four per thread.  us, quantize + unquantize:
+//                                    full items   1 CTA   2 CTAs   3 CTAs per SM
+//     1001 x  444  mean threshold       32.8       24.6     24.6     24.6
+//     2048 x  800  mean threshold       32.8       30.8     30.8     39.0
+//     1024 x 1024  mean threshold       24.7       22.6     22.6     26.7
+//     2048 x 2048  threshold 0          24.7       24.7     22.6     26.0
+//     2048 x 1323  4 bits               28.1       28.1     26.7     23.8
+//     2048 x  800  4 bits               26.7       22.6     20.6     22.6
+//    20000 x  400  threshold 0                               309      267
+static int balanced_cols(long long M, long long N, int mode, const LaunchCfg& cfg)
 {
-    if (N > (long long) fit * (cfg.numSMs - 1))
-        return fit;
-    const long long slots = (long long) cfg.numSMs * cfg.ctasPerSM;
-    long long c = (N + slots - 1) / slots;
-    if (c * M < 1024)
-        c = (1024 + M - 1) / M;
-    return (int) (c < fit ? c : fit);
+    bool resident = false;
+    const int fit = cols_per_item(M, N, cfg.smemFloats, &resident);
+    const long long least = (1024 + M - 1) / M;
+    auto dealt = [&](long long slots) { return std::min<long long>(fit, std::max((N + slots - 1) / slots, least)); };
+    auto perSM = [&](long long c) { return c * (((N + c - 1) / c + cfg.numSMs - 1) / cfg.numSMs); };
+    const long long two = dealt(2LL * cfg.numSMs);
+    const long long three = dealt(3LL * cfg.numSMs);
+    if (cfg.ctasPerSM < 3 || (resident && mode != MODE_MULTIBIT))
+        return (int) two;
+    if (!resident)
+        return (int) three;
+    return (int) (perSM(three) < perSM(two) || (perSM(three) == perSM(two) && (M & 3)) ? three : two);
 }
 
 void fill_layout(QTensor* t, long long M, long long N, int bits)
@@ -161,7 +174,7 @@ int qagg_quantize(void* stream, const float* grad, const float* res_in, float* r
     t.res_in = res_in;
     t.res_out = res_out;
     t.pk[0] = static_cast<unsigned char*>(packed);
-    const int c = balanced_cols(M, N, cols_per_item(M, N, cfg.smemFloats, nullptr), cfg);
+    const int c = balanced_cols(M, N, mode_of(bits, zero_threshold), cfg);
     const int nItems = (int) ((N + c - 1) / c);
     return check_cuda(launch_colquant((cudaStream_t) stream, false, mode_of(bits, zero_threshold), &t, nullptr, nullptr, nItems, c, cfg),
                       "quantize kernel launch");
@@ -218,7 +231,7 @@ int qagg_reduce_requantize(void* stream, const void* const* stripes, int K, cons
         if (!t.src[s] && !(s == 0 && self_raw))
             return fail(QAGG_EINVAL, "qagg_reduce_requantize: null stripe pointer");
     }
-    const int c = balanced_cols(M, n, cols_per_item(M, n, cfg.smemFloats, nullptr), cfg);
+    const int c = balanced_cols(M, n, mode_of(bits, zero_threshold), cfg);
     const int nItems = (int) ((n + c - 1) / c);
     return check_cuda(launch_colquant((cudaStream_t) stream, true, mode_of(bits, zero_threshold), &t, nullptr, nullptr, nItems, c, cfg),
                       "reduce-requantize kernel launch");

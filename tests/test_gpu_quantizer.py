@@ -109,9 +109,11 @@ def test_edge_shapes_bit_exact(G, oracle_port, shape, bits, zero_thr):
         G.assert_same_bits(G.host(out_g), out_o, f"{shape} b{bits} it{it} output")
 
 
-# columns per item: the most that still leave an SM without one (dealt over 444 CTA slots) and one more (full items), single
-# columns, the 1024-value floor, columns streamed in chunks
-@pytest.mark.parametrize("shape", [(2052, 1176), (2052, 1177), (1001, 444), (1001, 445), (5, 4096), (1, 445), (1023, 9), (20000, 13)], ids=lambda s: f"{s[0]}x{s[1]}")
+# columns per item on 148 SMs: one per item and the last count where that holds (296), two; as many as fit and the last count that
+# is dealt (9 x 296); three CTAs per SM at 4 bits (1323: 9 columns per SM instead of 10; 1001 x 2600: plain loads); the 1024-value
+# floor; columns streamed in chunks
+@pytest.mark.parametrize("shape", [(2052, 296), (2052, 297), (2052, 1323), (2052, 2664), (2052, 2665), (1001, 517), (1001, 2600), (5, 4096), (1, 445),
+                                   (1023, 9), (20000, 13)], ids=lambda s: f"{s[0]}x{s[1]}")
 @pytest.mark.parametrize("bits,zero_thr", [(1, True), (1, False), (4, True)])
 def test_dealt_columns_bit_exact(G, oracle_port, shape, bits, zero_thr):
     test_edge_shapes_bit_exact(G, oracle_port, shape, bits, zero_thr)
