@@ -101,30 +101,28 @@ __device__ __forceinline__ void pack_words(unsigned (&x)[PACK_ILP], int lane)
 // every chunk of the item has been fetched by then, and no other item uses these columns), so no unquantize launch follows and
 // the packed matrix is not read back.  A thread takes four consecutive rows of a column and stores them as one 16-byte
 // vector; threads are dealt to the item's rows column after column, so short columns keep all threads busy.
-__device__ __forceinline__ void expand_item(const QTensor& T, int col0, int nc, int Q, bool vec, const unsigned* bitmap, const float* lv0, const float* lv1)
+template <bool VEC>
+__device__ __forceinline__ void expand_columns(float* out, unsigned M, unsigned nc, unsigned Q, const unsigned* bitmap, const float* lv0, const float* lv1)
 {
-    const unsigned M = (unsigned) T.M;
-    float* const out = T.out + (size_t) col0 * M;
     // A column that is not 16-byte aligned has up to three rows before its first boundary and up to three after its last: they are
     // stored one by one, in up to six units after the quads (with one row per unit throughout, the last item of a 39997 x 13
     // matrix kept its CTA 25 us longer).
-    const unsigned units = vec ? M >> 2 : (M >> 2) + 6u; // per column
+    const unsigned units = VEC ? M >> 2 : (M >> 2) + 6u; // per column
     const unsigned advC = NT / units, advU = NT - advC * units;
     unsigned c = threadIdx.x / units, u = threadIdx.x - c * units;
 #pragma unroll 4
-    while (c < (unsigned) nc)
+    while (c < nc)
     {
-        const unsigned* const bits = bitmap + c * (unsigned) (Q + 1);
+        const unsigned* const bits = bitmap + c * (Q + 1);
         const float v0 = lv0[c], v1 = lv1[c];
-        if (vec)
+        float* const o = out + (size_t) c * M;
+        if (VEC)
         {
             const unsigned b = bits[u >> 3] >> (4u * (u & 7u));
-            __stcs(reinterpret_cast<float4*>(out + (size_t) c * M) + u,
-                   make_float4((b & 1u) ? v1 : v0, (b & 2u) ? v1 : v0, (b & 4u) ? v1 : v0, (b & 8u) ? v1 : v0));
+            __stcs(reinterpret_cast<float4*>(o) + u, make_float4((b & 1u) ? v1 : v0, (b & 2u) ? v1 : v0, (b & 4u) ? v1 : v0, (b & 8u) ? v1 : v0));
         }
         else
         {
-            float* const o = out + (size_t) c * M;
             const unsigned head = min(M, (4u - ((unsigned) (reinterpret_cast<uintptr_t>(o) >> 2) & 3u)) & 3u);
             const unsigned quads = (M - head) >> 2;
             if (u < quads)
@@ -149,6 +147,15 @@ __device__ __forceinline__ void expand_item(const QTensor& T, int col0, int nc, 
             ++c;
         }
     }
+}
+__device__ __forceinline__ void expand_item(const QTensor& T, int col0, int nc, int Q, bool vec, const unsigned* bitmap, const float* lv0, const float* lv1)
+{
+    const unsigned M = (unsigned) T.M;
+    float* const out = T.out + (size_t) col0 * M;
+    if (vec)
+        expand_columns<true>(out, M, (unsigned) nc, (unsigned) Q, bitmap, lv0, lv1);
+    else
+        expand_columns<false>(out, M, (unsigned) nc, (unsigned) Q, bitmap, lv0, lv1);
 }
 
 template <bool EXPAND>
