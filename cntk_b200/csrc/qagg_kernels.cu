@@ -439,15 +439,15 @@ __device__ __forceinline__ unsigned quant_one(const ValQ& q, int bits, float val
     return bit ? 1u : 0u;
 }
 
-template <int MODE>
+template <int MODE, bool EXPAND>
 __device__ __forceinline__ void quantize_resident(const QTensor& T, const Signal& sg, int col0, int nc, int stride, const float* __restrict__ smem,
-                                                  const ColStats& S, bool expand)
+                                                  const ColStats& S)
 {
     const int M = (int) T.M;
     const int Q = T.Q;
     const int bits = T.bits;
     const int vpw = 32 / bits;
-    float* const outBase = expand ? T.out : nullptr;
+    float* const outBase = EXPAND ? T.out : nullptr;
     const bool vec = ((Q & 3) == 0) && ((M & 3) == 0) && ((reinterpret_cast<uintptr_t>(T.res_out) & 15) == 0) &&
                      ((reinterpret_cast<uintptr_t>(outBase) & 15) == 0);
     if (vec)
@@ -486,7 +486,7 @@ __device__ __forceinline__ void quantize_resident(const QTensor& T, const Signal
                 w2 |= quant_one<MODE>(q, bits, val0, val1, v.z, r.z, x.z) << sh;
                 w3 |= quant_one<MODE>(q, bits, val0, val1, v.w, r.w, x.w) << sh;
                 __stcs(reinterpret_cast<float4*>(rp + k * Q), r);
-                if (outBase)
+                if (EXPAND)
                     __stcs(reinterpret_cast<float4*>(op + k * Q), x);
             }
             const unsigned ws[4] = {w0, w1, w2, w3};
@@ -522,7 +522,7 @@ __device__ __forceinline__ void quantize_resident(const QTensor& T, const Signal
                 float r, x;
                 word |= quant_one<MODE>(q, bits, val0, val1, vp[k * Q], r, x) << (k * bits);
                 rp[k * Q] = r;
-                if (outBase)
+                if (EXPAND)
                     op[k * Q] = x;
             }
             store_words(T, sg, j, w, &word, 1, lower, upper);
@@ -534,8 +534,8 @@ __device__ __forceinline__ void quantize_resident(const QTensor& T, const Signal
 // compiler keeps every load behind the stores before it; AHEAD rows of a word are therefore loaded before the first of them is
 // stored (39997 x 13 at 4 bits: 198 us per step, 223 one row at a time; 8 rows ahead measured the same at 4 bits, but the kernel
 // then spills and eight 1024 x 1024 at 4 bits, which never come here, went from 41.9 to 45.9 us).
-template <int MODE, bool STRIPES>
-__device__ __forceinline__ void quantize_streamed(const QTensor& T, const Signal& sg, int col0, int nc, const ColStats& S, bool expand)
+template <int MODE, bool STRIPES, bool EXPAND>
+__device__ __forceinline__ void quantize_streamed(const QTensor& T, const Signal& sg, int col0, int nc, const ColStats& S)
 {
     const int M = (int) T.M;
     const int Q = T.Q;
@@ -552,7 +552,7 @@ __device__ __forceinline__ void quantize_streamed(const QTensor& T, const Signal
         const ValQ q = make_valq(bits, lower, upper);
         const float val0 = unquantize_val(q, 1, 0u), val1 = unquantize_val(q, 1, 1u);
         float* rp = T.res_out + (size_t) j * M + w;
-        float* op = expand ? T.out + (size_t) j * M + w : nullptr;
+        float* op = EXPAND ? T.out + (size_t) j * M + w : nullptr;
         const int nk = min(vpw, (M - w + Q - 1) / Q);
         unsigned word = 0;
         for (int k0 = 0; k0 < nk; k0 += AHEAD)
@@ -570,7 +570,7 @@ __device__ __forceinline__ void quantize_streamed(const QTensor& T, const Signal
                 float r, x;
                 word |= quant_one<MODE>(q, bits, val0, val1, v[u], r, x) << (k * bits);
                 rp[(size_t) k * Q] = r;
-                if (op)
+                if (EXPAND)
                     op[(size_t) k * Q] = x;
             }
         }
@@ -583,20 +583,20 @@ __device__ __forceinline__ void quantize_streamed(const QTensor& T, const Signal
 //   A. all threads stage the columns' fp32 values in shared memory (one coalesced pass over the inputs);
 //   B. the columns are walked in row order and each column's range is derived;
 //   C. all threads quantize, pack words, write the residual and the packed column to its owner's buffer.
-// `expand` (one rank: nothing is added to what this rank quantized): phase C also stores what each field unquantizes to into
+// EXPAND (one rank: nothing is added to what this rank quantized): phase C also stores what each field unquantizes to into
 // T.out, which may be the gradient itself (a column's inputs are read before its phase C, by the same CTA), and no
 // unquantize launch follows.  The kernel waits for add chains, not for memory, so the extra 4 bytes per value ride along.
 // Several CTAs are resident per SM, so one CTA's walk overlaps the others' memory phases.  Work items are
 // handed out through a global counter (tallest columns first) when `counters` is given.
 // Columns too tall to stage are streamed through shared memory in chunks for B and re-read for C.
 // =================================================================================================================
-template <bool STRIPES, int MODE, bool TABLE>
+template <bool STRIPES, int MODE, bool TABLE, bool EXPAND>
 #ifndef QAGG_CTAS_PER_SM
 #define QAGG_CTAS_PER_SM 3 // resident CTAs per SM the column kernel is compiled and configured for
 #endif
 __global__ void __launch_bounds__(NT, QAGG_CTAS_PER_SM) k_colquant(const QTensor single, const QTensor* __restrict__ tensors,
                                                     const QItem* __restrict__ items, int nItems, int colsPerItem, int smemFloats,
-                                                    int numSMs, unsigned* __restrict__ counters, const Signal signal, int expand)
+                                                    int numSMs, unsigned* __restrict__ counters, const Signal signal)
 {
     extern __shared__ __align__(16) float smem[];
     __shared__ QTensor sT;
@@ -699,7 +699,7 @@ __global__ void __launch_bounds__(NT, QAGG_CTAS_PER_SM) k_colquant(const QTensor
                 }
                 __syncthreads();
             }
-            quantize_resident<MODE>(T, signal, col0, nc, stride, smem, S, TABLE && !STRIPES && expand);
+            quantize_resident<MODE, EXPAND>(T, signal, col0, nc, stride, smem, S);
         }
         else
         {
@@ -750,7 +750,7 @@ __global__ void __launch_bounds__(NT, QAGG_CTAS_PER_SM) k_colquant(const QTensor
                 S.upper[lane] = up;
             }
             __syncthreads();
-            quantize_streamed<MODE, STRIPES>(T, signal, col0, nc, S, TABLE && !STRIPES && expand);
+            quantize_streamed<MODE, STRIPES, EXPAND>(T, signal, col0, nc, S);
         }
     }
     // The last CTA to leave re-arms the work counter for the next launch and, if asked to, tells the peers that every
@@ -831,11 +831,11 @@ int cols_per_item(long long M, long long N, int smemFloats, bool* resident, int 
     return (int) c;
 }
 
-template <bool STRIPES, int MODE, bool TABLE>
+template <bool STRIPES, int MODE, bool TABLE, bool EXPAND>
 static cudaError_t launch_cq(cudaStream_t st, const QTensor* single, const QTensor* tensors, const QItem* items,
-                             int nItems, int colsPerItem, const LaunchCfg& cfg, unsigned* counters, const Signal& signal, bool expand)
+                             int nItems, int colsPerItem, const LaunchCfg& cfg, unsigned* counters, const Signal& signal)
 {
-    auto kern = k_colquant<STRIPES, MODE, TABLE>;
+    auto kern = k_colquant<STRIPES, MODE, TABLE, EXPAND>;
     const size_t smemBytes = (size_t) cfg.smemFloats * sizeof(float);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smemBytes);
     if (e != cudaSuccess)
@@ -844,7 +844,7 @@ static cudaError_t launch_cq(cudaStream_t st, const QTensor* single, const QTens
     if (grid > nItems)
         grid = nItems;
     static const QTensor zero = {};
-    kern<<<grid, NT, smemBytes, st>>>(single ? *single : zero, tensors, items, nItems, colsPerItem, cfg.smemFloats, cfg.numSMs, counters, signal, expand ? 1 : 0);
+    kern<<<grid, NT, smemBytes, st>>>(single ? *single : zero, tensors, items, nItems, colsPerItem, cfg.smemFloats, cfg.numSMs, counters, signal);
     return cudaGetLastError();
 }
 
@@ -962,21 +962,20 @@ cudaError_t launch_colquant(cudaStream_t st, bool stripes, int mode, const QTens
         return cudaSuccess;
     }
     const bool table = (single == nullptr);
-#define QAGG_CASE(S, MD, TB) \
-    if (stripes == S && mode == MD && table == TB) \
-        return launch_cq<S, MD, TB>(st, single, tensors, items, nItems, colsPerItem, cfg, counters, signal, expand);
-    QAGG_CASE(false, MODE_ONEBIT_ZERO, false)
-    QAGG_CASE(false, MODE_ONEBIT_MEAN, false)
-    QAGG_CASE(false, MODE_MULTIBIT, false)
-    QAGG_CASE(true, MODE_ONEBIT_ZERO, false)
-    QAGG_CASE(true, MODE_ONEBIT_MEAN, false)
-    QAGG_CASE(true, MODE_MULTIBIT, false)
-    QAGG_CASE(false, MODE_ONEBIT_ZERO, true)
-    QAGG_CASE(false, MODE_ONEBIT_MEAN, true)
-    QAGG_CASE(false, MODE_MULTIBIT, true)
-    QAGG_CASE(true, MODE_ONEBIT_ZERO, true)
-    QAGG_CASE(true, MODE_ONEBIT_MEAN, true)
-    QAGG_CASE(true, MODE_MULTIBIT, true)
+    expand = expand && table && !stripes;
+#define QAGG_CASE(S, MD, TB, EX) \
+    if (stripes == S && mode == MD && table == TB && expand == EX) \
+        return launch_cq<S, MD, TB, EX>(st, single, tensors, items, nItems, colsPerItem, cfg, counters, signal);
+#define QAGG_CASES(MD) \
+    QAGG_CASE(false, MD, false, false) \
+    QAGG_CASE(false, MD, true, false) \
+    QAGG_CASE(false, MD, true, true) \
+    QAGG_CASE(true, MD, false, false) \
+    QAGG_CASE(true, MD, true, false)
+    QAGG_CASES(MODE_ONEBIT_ZERO)
+    QAGG_CASES(MODE_ONEBIT_MEAN)
+    QAGG_CASES(MODE_MULTIBIT)
+#undef QAGG_CASES
 #undef QAGG_CASE
     return cudaErrorInvalidValue;
 }
