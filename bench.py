@@ -14,13 +14,15 @@ columns of every tensor of one more full-size step is replayed through the whole
 more than one rank the small multi-rank parity set of tests/multi_gpu_check.py runs as well.  A differing byte ends the
 process with a non-zero status; the line carries "parity": {"checked": true, ...}.
 
---impl reference times the reference's own CPU quantizer (its headers compiled in place, oracle/_ref; else the C port)
-driving the restated exchange with one thread per simulated rank on this box's host cores, and prints the same line shape.
+--impl reference times the reference's own CPU quantizer (its headers compiled in place, oracle/_ref) driving the restated
+exchange with one thread per simulated rank on this box's host cores, and prints the same line shape; where that build is
+missing it prints why there is no such arm.  (The C restatement of the quantizer is no stand-in for it: it is only timed as
+"cpu_baseline" of this build's own line, under its own name.)
 --local-ranks K (one GPU) steps K simulated ranks as an in-process group and prints each rank's kernel times per phase: the way
 to look at the owner's reduce-requantize kernels, which a single rank never runs, on one device and under a profiler.  Its
 line is a kernel-time table, not a bench value.  --fused-update adds the learner step (momentum SGD) fused into the last
 kernel beside the unfused sequence.
---workload sweep runs BASELINE config 5 (1024 rows x 1 Mi .. 1 Gi values; 1, 2 and 32 bits) and reports a table in "sweep".
+--workload sweep runs the bandwidth sweep (1024 rows x 1 Mi .. 1 Gi values; 1, 2 and 32 bits) and reports a table in "sweep".
 """
 import argparse
 import json
@@ -96,10 +98,10 @@ class ClockSampler:
                 "reasons": sorted(reasons), "samples": len(sm)}
 
 
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of ONE launch of the quantize kernel at ONE rank, from the ncu
-# capture summarised in profiles/k_stream1_speech_dnn_1bit.md (same workload).  Reported only for the configuration that
-# was captured; null elsewhere.
-NCU_TRAFFIC_BYTES = {("speech_dnn", 1): 504.58e6}
+# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of ONE launch of the quantize kernel at ONE rank, which expands
+# too, from the ncu capture of this workload that is summarised under profiles/.  Reported only for the configuration that was
+# captured; null elsewhere.
+NCU_TRAFFIC_BYTES = {("speech_dnn", 1): 670.92e6}
 
 
 def get_shapes(name):
@@ -177,6 +179,11 @@ def workload_config(workload, shapes, V, bits, K):
 def run_reference(args):
     rank, _, world = dist_env()
     if rank != 0:
+        return
+    from oracle import backend
+    if not backend.have_ref():
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's quantizer headers are not built here (oracle/_ref needs a CNTK checkout)"}),
+              flush=True)
         return
     shapes, bits = get_shapes(args.workload if args.workload != "sweep" else "speech_dnn")
     K = args.gpus
@@ -439,12 +446,13 @@ def run_ours(args):
                 d.update(extra)
             return d
 
-        k1 = roof("quantize", "k_stream1 (quantize: level sums + pack + deferred residual)", phases[0])
+        name = "k_stream1 (quantize: level sums + pack + deferred residual)" if bits == 1 else "k_colquant (quantize: range + pack + residual)"
+        k1 = roof("quantize", name if K > 1 else name[:-1] + " + unquantized values)", phases[0])
         kern_ms = phases[0] + phases[2] + phases[4]
         roofline = {"bound": "hbm", "kernel": k1["kernel"], "achieved": k1["achieved"], "peak": peak, "unit": "GB/s", "frac": k1["frac"],
                     "peak_kind": peak_kind, "traffic": NCU_TRAFFIC_BYTES.get((args.workload, K)),
                     "algorithmic_bytes_per_launch": alg["quantize"],
-                    "unquantize": roof("unquantize", "k_unquantize", phases[4]),
+                    "unquantize": roof("unquantize", "k_unquantize", phases[4]) if K > 1 else None,
                     "all_kernels": {"algorithmic_bytes": alg["total"], "ms": kern_ms,
                                     "frac": alg["total"] / (kern_ms * 1e-3) / 1e9 / peak if kern_ms > 0 else None}}
         if K > 1:
@@ -485,7 +493,7 @@ def run_ours(args):
 
 
 def run_sweep(args):
-    """one 1024-row matrix of 1 Mi .. 1 Gi values; 1 bit, 2 bits and the unquantized 32-bit arm; at the
+    """Bandwidth sweep: one 1024-row matrix of 1 Mi .. 1 Gi values; 1 bit, 2 bits and the unquantized 32-bit arm; at the
     launched number of ranks.  One JSON line with the table under "sweep"."""
     import torch
     from cntk_b200 import lib, workloads
@@ -600,9 +608,9 @@ def run_local_group(args):
            "workload": args.workload, "bits": bits, "steps": args.steps, "warmup": args.warmup,
            "quantize_us": k1, "reduce_requantize_us": k2, "unquantize_us": k3,
            "roofline_frac_of_" + peak_kind: {
-               "quantize": round((12 * V + P) / (max(k1) * 1e-6) / (peak * 1e9), 3),
+               "quantize": round(((12 if K > 1 else 16) * V + P) / (max(k1) * 1e-6) / (peak * 1e9), 3),
                "reduce_requantize": round((8 * V / K + P * (1 + 1.0 / K)) / (max(k2) * 1e-6) / (peak * 1e9), 3) if K > 1 else None,
-               "unquantize": round((4 * V + P) / (max(k3) * 1e-6) / (peak * 1e9), 3)}}
+               "unquantize": round((4 * V + P) / (max(k3) * 1e-6) / (peak * 1e9), 3) if K > 1 else None}}
     if args.fused_update:
         w = [[torch.randn_like(t) for t in pool] for _ in range(K)]
         sm = [[torch.zeros_like(t) for t in pool] for _ in range(K)]
@@ -634,8 +642,12 @@ def run_local_group(args):
         rank_update_ms(True)  # switches the fused step on (and warms it up)
         ph_f = timed(args.steps)
         k3_fused = max(p_[4] for p_ in ph_f)
+        if K == 1:
+            # the unfused step unquantizes inside the quantize kernel: what that adds to the kernel is its unquantize time
+            k3_plain = max(0.0, max(k1) * 1e-3 - max(p_[0] for p_ in ph_f))
         out["consumer_fusion"] = {"rule": "momentum SGD (Matrix::MomentumSGDUpdate)", "unfused_ms": round(k3_plain + unf, 4),
-                                  "unfused_parts_ms": {"unquantize": round(k3_plain, 4), "update_kernels": round(unf, 4)},
+                                  "unfused_parts_ms": {"unquantize" if K > 1 else "unquantize_inside_quantize": round(k3_plain, 4),
+                                                       "update_kernels": round(unf, 4)},
                                   "fused_ms": round(k3_fused, 4),
                                   "bytes_unfused": 24 * V + P, "bytes_fused": 16 * V + P,
                                   "fused_frac_of_" + peak_kind: round((16 * V + P) / (k3_fused * 1e-3) / (peak * 1e9), 3)}

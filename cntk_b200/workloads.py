@@ -62,10 +62,11 @@ def packed_bytes(shapes, bits):
 
 def algorithmic_bytes(shapes, bits, K):
     """Bytes one rank must move through HBM per step when every input and output is touched exactly once:
-    quantize 12V + P, owner reduce 8V/K + P(1 + 1/K), unquantize 4V + P  (V values, P packed bytes)."""
+    quantize 12V + P, owner reduce 8V/K + P(1 + 1/K), unquantize 4V + P  (V values, P packed bytes).  With one rank the
+    quantize kernel stores the unquantized values too and nothing reads the packed matrix: quantize 16V + P."""
     V, P = total_values(shapes), packed_bytes(shapes, bits)
-    k1 = 12 * V + P
-    k3 = 4 * V + P
+    k1 = (16 if K == 1 else 12) * V + P
+    k3 = 0 if K == 1 else 4 * V + P
     k2 = 0 if K == 1 else 8 * V / K + P * (1 + 1 / K)
     return {"quantize": k1, "reduce_requantize": k2, "unquantize": k3, "total": k1 + k2 + k3}
 

@@ -91,8 +91,7 @@ int qagg_reduce_requantize(void* stream, const void* const* stripes, int K, cons
 /* The same three for ElemType = double (MatrixQuantizerImpl<double>; QWord = unsigned long long, Source/Math/ValueQuantizer.h:48-55):
  * a packed column is `double lower; double upper; uint64 words[Q]`, Q = ceil(M*bits/64), 64 one-bit values per word, bits a
  * power of two in 1..64 (64 = bit-cast pass-through).  Bit-identical to the reference CPU quantizer instantiated for double
- * (what its own 1-bit end-to-end tests run, precision=double).  Buffers must be 8-byte aligned.  The striped aggregator is
- * float only. */
+ * (what its own 1-bit end-to-end tests run, precision=double).  Buffers must be 8-byte aligned. */
 int64_t qagg_packed_col_bytes_f64(int64_t M, int bits);
 int64_t qagg_packed_bytes_f64(int64_t M, int64_t N, int bits);
 int qagg_quantize_f64(void* stream, const double* grad, const double* res_in, double* res_out, void* packed,
@@ -358,7 +357,8 @@ int qagg_wait_flags(void* stream, const unsigned* flags_dev, int n, int skip, un
  * "Actual gradient aggregation time" trace, AllReduceDistGradAggregator.h:241-246, 560-565).  When enabled, each step records
  * CUDA events on its stream around its five phases.  qagg_agg_phase_ms waits for the recorded steps and returns the mean
  * milliseconds per step, over the (at most 64) most recent steps since the last read, for
- * {quantize, scatter, reduce-requantize, all-gather, unquantize} (about 0 for phases a 1-rank step skips). */
+ * {quantize, scatter, reduce-requantize, all-gather, unquantize} (about 0 for phases a 1-rank step skips: all but quantize,
+ * which then writes the aggregated gradients too, and unquantize while a learner step is bound or gradients share memory). */
 int qagg_agg_set_profiling(qagg_aggregator* a, int enabled);
 int qagg_agg_phase_ms(qagg_aggregator* a, float* out5);
 /* Bytes one step sends over the wire from this rank (scatter + gather), and kernels it launches. */
