@@ -494,7 +494,8 @@ def _same_or_both_nan(a, b, what):
     assert ok.all(), f"{what}: {int((~ok).sum())} of {a.size} elements differ (NaN positions must agree, everything else bit for bit)"
 
 
-@pytest.mark.parametrize("K,tall_rows,zero_thr", [(1, None, True), (3, None, True), (3, "200", True), (2, "0", True), (2, None, False)])
+@pytest.mark.parametrize("K,tall_rows,zero_thr", [(1, None, True), (3, None, True), (3, "200", True), (2, "0", True), (2, None, False),
+                                                  (1, "200", True), (1, None, False)])
 def test_nan_and_infinities_spread_like_the_reference(G, oracle_port, K, tall_rows, zero_thr, monkeypatch):
     """A NaN (or a pair of opposite infinities) in a gradient makes its column's range NaN in the reference
     (ColumnQuantizer.h:247-316: the value lands in the upper partition sum), its bit 0, and its residual NaN from then on;

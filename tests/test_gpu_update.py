@@ -150,3 +150,12 @@ def test_fused_update_behind_the_form_walk_quantize_path(G, oracle_port, monkeyp
     every matrix with 2048 rows or more, the streaming kernel the others."""
     monkeypatch.setenv("QAGG_TALL_ROWS", "2048")
     test_aggregator_fused_update(G, oracle_port, 4, 1, True)
+
+
+def test_fused_update_and_expansion_take_turns_on_one_rank(G, oracle_port, monkeypatch):
+    """With one rank a step without the update is expanded by the kernels that quantize (tall matrices by a launch of their own),
+    a step with it by the unquantize-update launch: the state carries over in both directions."""
+    monkeypatch.setenv("QAGG_TALL_ROWS", "2048")
+    test_aggregator_fused_update(G, oracle_port, 1, 1, False)
+    monkeypatch.delenv("QAGG_TALL_ROWS")
+    test_aggregator_fused_update(G, oracle_port, 1, 8, False)
