@@ -447,6 +447,8 @@ __device__ __forceinline__ void quantize_resident(const QTensor& T, const Signal
     const int Q = T.Q;
     const int bits = T.bits;
     const int vpw = 32 / bits;
+    // (tested where it is stored through, although it is never null with EXPAND: without the test the mean-threshold instantiation
+    // is scheduled worse, 115 -> 131 us for a set around a 3664 x 3664 matrix)
     float* const outBase = EXPAND ? T.out : nullptr;
     const bool vec = ((Q & 3) == 0) && ((M & 3) == 0) && ((reinterpret_cast<uintptr_t>(T.res_out) & 15) == 0) &&
                      ((reinterpret_cast<uintptr_t>(outBase) & 15) == 0);
@@ -486,7 +488,7 @@ __device__ __forceinline__ void quantize_resident(const QTensor& T, const Signal
                 w2 |= quant_one<MODE>(q, bits, val0, val1, v.z, r.z, x.z) << sh;
                 w3 |= quant_one<MODE>(q, bits, val0, val1, v.w, r.w, x.w) << sh;
                 __stcs(reinterpret_cast<float4*>(rp + k * Q), r);
-                if (EXPAND)
+                if (outBase)
                     __stcs(reinterpret_cast<float4*>(op + k * Q), x);
             }
             const unsigned ws[4] = {w0, w1, w2, w3};
@@ -522,7 +524,7 @@ __device__ __forceinline__ void quantize_resident(const QTensor& T, const Signal
                 float r, x;
                 word |= quant_one<MODE>(q, bits, val0, val1, vp[k * Q], r, x) << (k * bits);
                 rp[k * Q] = r;
-                if (EXPAND)
+                if (outBase)
                     op[k * Q] = x;
             }
             store_words(T, sg, j, w, &word, 1, lower, upper);
